@@ -40,7 +40,7 @@ TRAFFIC_RECORD = os.path.join(ROOT, "profiles", "conv_i8_tc_kernel_config1.md")
 
 def ncu_traffic_record():
     """DRAM bytes per convolution launch from the ncu capture summarised under profiles/, valid only for the kernel source
-    it was captured with: the summary carries the SHA-256 of tennis_b200/csrc/conv_tc.cu at capture time.  Returns
+    it was captured with: the summary carries the SHA-256 of tennis_b200/csrc/conv_tc_kernel.cuh at capture time.  Returns
     (bytes or None, stale flag, note)."""
     import hashlib
     import re
@@ -50,7 +50,7 @@ def ncu_traffic_record():
         m_hash = re.search(r"conv_tc_sha256\s*=\s*([0-9a-f]{64})", text)
         if not m_bytes or not m_hash:
             return None, True, "no traffic record in %s" % os.path.relpath(TRAFFIC_RECORD, ROOT)
-        now = hashlib.sha256(open(os.path.join(ROOT, "tennis_b200", "csrc", "conv_tc.cu"), "rb").read()).hexdigest()
+        now = hashlib.sha256(open(os.path.join(ROOT, "tennis_b200", "csrc", "conv_tc_kernel.cuh"), "rb").read()).hexdigest()
         if now != m_hash.group(1):
             return None, True, "the kernel source changed since the ncu capture in %s" % os.path.relpath(TRAFFIC_RECORD, ROOT)
         return float(m_bytes.group(1)), False, "ncu capture summarised in %s" % os.path.relpath(TRAFFIC_RECORD, ROOT)

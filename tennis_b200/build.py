@@ -6,7 +6,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 
 
 def build(verbose=False):
-    cmd = ["make", "-C", os.path.join(_HERE, "csrc"), "-j4"]
+    cmd = ["make", "-C", os.path.join(_HERE, "csrc"), "-j8"]
     out = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if verbose or out.returncode != 0:
         print(out.stdout)
