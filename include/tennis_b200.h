@@ -237,7 +237,7 @@ TSB_API int tsb_conv2d_i8_run(tsb_conv_plan *plan, const int8_t *x, int x_layout
  * NULL; residual_after_activation keeps its meaning).  Every fp32 step is rounded separately, as when the projection is
  * run on its own and handed over as a residual tensor, so the results are the same bits; the projection's fp32 output is
  * never written to or read from global memory.  Both inputs are NHWC_PAD int8, 16-byte aligned; the outputs are
- * pixel-major fp32 and / or NHWC_PAD int8 with half-away rounding (one requantize scale or one per image); both plans
+ * pixel-major fp32 and / or NHWC_PAD int8 (one requantize scale for the batch or one per image); both plans
  * have had tsb_conv2d_i8_set_weights.  shortcut_dequantize_scales and shortcut_bias are device arrays of O floats.
  * tile_channels: 0 = the library chooses, 128 or 256 = output channels per tile (a tuning override for tests).
  * Returns TSB_ERR_UNSUPPORTED for anything else; the caller then runs the two convolutions one after the other.

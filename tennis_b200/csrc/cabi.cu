@@ -323,7 +323,7 @@ static int build_epilogue(const tsb_conv_plan *plan, const tsb_conv_epilogue *e,
     p.out_cp = tsb_padded_channels(g.O);
     p.O = g.O;
     p.P = g.OH * g.OW;
-    p.rne_limit = 0; p.group_len = 1; p.nscales = 1;
+    p.rne_limit = 0; p.even = 0; p.tail = 0; p.group_len = 1; p.nscales = 1;
     p.rq_scales[0] = 1.0f;
     if (e->out_i8) {
         if (!e->requant_scales_host || e->n_requant_scales < 1) return fail(TSB_ERR_INVALID_ARGUMENT, "run: out_i8 needs requantize scales");
@@ -331,6 +331,8 @@ static int build_epilogue(const tsb_conv_plan *plan, const tsb_conv_epilogue *e,
         if (p.i8_nhwc && reinterpret_cast<uintptr_t>(e->out_i8) % 16) return fail(TSB_ERR_INVALID_ARGUMENT, "run: NHWC out_i8 must be 16-byte aligned");
         QuantRule r = make_quant_rule((int64_t)g.N * g.O * g.OH * g.OW, e->n_requant_scales);
         p.rne_limit = (uint32_t)r.rne_limit;
+        p.even = r.rne_limit > 0;
+        p.tail = p.even && r.rne_limit < (int64_t)g.N * g.O * g.OH * g.OW;
         p.group_len = (uint32_t)r.group_len;
         p.nscales = r.nscales;
         for (int i = 0; i < e->n_requant_scales; ++i) p.rq_scales[i] = e->requant_scales_host[i];

@@ -34,6 +34,8 @@ struct EpiParams {
     int O, P;           // output channels, OH*OW
     // requantize
     uint32_t rne_limit;
+    int even;           // half-to-even (one scale), but for the elements from rne_limit on; 0: half away from zero everywhere
+    int tail;           // there are such elements (the tensor's count is no multiple of eight)
     uint32_t group_len;
     int nscales;
     float rq_scales[kMaxRequantScales];

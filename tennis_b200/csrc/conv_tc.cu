@@ -9,8 +9,8 @@
 namespace tsb {
 namespace tc {
 
-#define TSB_TC_EXTERN(BN_, BK_, SWAP_, MODE_, DUAL_)                                                                         \
-    extern template int launch<BN_, BK_, SWAP_, MODE_, DUAL_>(const Config &, const CUtensorMap &, const CUtensorMap &,     \
+#define TSB_TC_EXTERN(BN_, BK_, SWAP_, MODE_, EPI_, DUAL_)                                                                         \
+    extern template int launch<BN_, BK_, SWAP_, MODE_, EPI_, DUAL_>(const Config &, const CUtensorMap &, const CUtensorMap &,     \
                                                               const CUtensorMap &, const CUtensorMap &, const CUtensorMap &, \
                                                               const KernelParams &, const EpiParams &, cudaStream_t,         \
                                                               const std::conditional_t<DUAL_, DualParams, NoDual> &);
@@ -123,7 +123,7 @@ int staging_level(const View &v, const EpiParams &epi) {
     const ConvGeom &g = v.real;
     if (epi.out_acc) return 0;
     const bool per_sample = epi.nscales > 1 && epi.nscales == g.N && epi.group_len == (uint32_t)(g.O * g.OH * g.OW);
-    if (epi.out_i8 && !(epi.i8_nhwc && epi.rne_limit == 0 && (epi.nscales == 1 || per_sample))) return 0;
+    if (epi.out_i8 && !(epi.i8_nhwc && (epi.nscales == 1 || per_sample))) return 0;
     if (epi.out_i8 && reinterpret_cast<uintptr_t>(epi.out_i8) % 16) return 0;
     const bool f32_tiles = (epi.out_f32 || epi.residual) && epi.f32_nhwc;
     if (f32_tiles) {
@@ -462,11 +462,11 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
     const ConvGeom &g = v.g;
     if (dual) {
         // the projected-shortcut kernels exist for the staged block epilogue only
-        const bool i8_ok = !epi.out_i8 || (epi.i8_nhwc && epi.rne_limit == 0 && reinterpret_cast<uintptr_t>(epi.out_i8) % 16 == 0 &&
+        const bool i8_ok = !epi.out_i8 || (epi.i8_nhwc && reinterpret_cast<uintptr_t>(epi.out_i8) % 16 == 0 &&
                                            (epi.nscales == 1 || (epi.nscales == g.N && epi.group_len == (uint32_t)(g.O * g.OH * g.OW))));
         const bool f32_ok = !epi.out_f32 || (epi.f32_nhwc && reinterpret_cast<uintptr_t>(epi.out_f32) % 16 == 0);
         if (epi.out_acc || epi.residual || !i8_ok || !f32_ok || g.O % 4 != 0 || cfg.swap || cfg.patch || v.rows || v.fold || cfg.staging != 2)
-            return fail(TSB_ERR_UNSUPPORTED, "projected shortcut: needs pixel-major fp32 / NHWC_PAD int8 outputs with half-away rounding, no residual tensor, O %% 4 == 0");
+            return fail(TSB_ERR_UNSUPPORTED, "projected shortcut: needs pixel-major fp32 / NHWC_PAD int8 outputs, no residual tensor, O %% 4 == 0");
     }
     KernelParams kp;
     kp.M_total = g.N * g.OH * g.OW;
@@ -508,24 +508,24 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
     }
     if (cfg.dyn_smem > kMaxDynamicSmem) return fail(TSB_ERR_UNSUPPORTED, "shared-memory plan of %u bytes does not fit", cfg.dyn_smem);
     const bool plain = !epi.out_acc && !epi.residual;
-    kp.epi_mode = kEpiGeneric;
-    if (plain && epi.out_f32 && !epi.f32_nhwc && !epi.out_i8) kp.epi_mode = kEpiF32Nchw;
+    int epi_mode = kEpiGeneric;      // which epilogue class the outputs take
+    if (plain && epi.out_f32 && !epi.f32_nhwc && !epi.out_i8) epi_mode = kEpiF32Nchw;
     // ... and with an fp32 NCHW residual (a shortcut folded into the convolution by the graph rewrite), where a thread owns a pixel
     if (!cfg.swap && !epi.out_acc && epi.residual && epi.out_f32 && !epi.f32_nhwc && !epi.out_i8 && (const void *)epi.residual != (const void *)epi.out_f32)
-        kp.epi_mode = kEpiF32Nchw;
-    const bool i8_fast = !epi.out_i8 || (epi.i8_nhwc && epi.rne_limit == 0 && (epi.nscales == 1 || kp.per_sample_scale));
-    if (plain && epi.out_i8 && !epi.out_f32 && i8_fast) kp.epi_mode = kEpiI8Nhwc;
-    // pixel-major fp32 tensors (block outputs and residuals of a network): 16-byte accesses need O % 4 == 0
-    if (!epi.out_acc && (epi.out_f32 || epi.residual) && epi.f32_nhwc && i8_fast && (const void *)epi.residual != (const void *)epi.out_f32 &&
-        (cfg.swap || (g.O % 4 == 0 && ((reinterpret_cast<uintptr_t>(epi.out_f32) | reinterpret_cast<uintptr_t>(epi.residual)) & 15) == 0)))
-        kp.epi_mode = kEpiNhwc;
+        epi_mode = kEpiF32Nchw;
+    const bool i8_fast = !epi.out_i8 || (epi.i8_nhwc && (epi.nscales == 1 || kp.per_sample_scale));
+    if (plain && epi.out_i8 && !epi.out_f32 && i8_fast) epi_mode = kEpiI8Nhwc;
+    // pixel-major fp32 tensors (block outputs and residuals of a network) where a thread owns a channel; where it owns a pixel they
+    // take the staged class, below
+    if (!epi.out_acc && (epi.out_f32 || epi.residual) && epi.f32_nhwc && i8_fast && (const void *)epi.residual != (const void *)epi.out_f32 && cfg.swap && !cfg.patch)
+        epi_mode = kEpiNhwc;
     const int mode = cfg.patch ? kModePatch : (v.rows ? kModeRows : kModeGeneral);
     // Pixel-major fp32 residual (the shortcut of a residual block, as large as the output): a tensor map over it lets the
     // epilogue prefetch the boxes it is about to read into L2.  The map is not used for loads, so a failure to encode one
     // only switches the prefetch off.
     CUtensorMap map_r = map_b;
     kp.res_prefetch = 0;
-    if (kp.epi_mode == kEpiNhwc && epi.residual && mode == kModeGeneral && g.O % 4 == 0 && reinterpret_cast<uintptr_t>(epi.residual) % 16 == 0 &&
+    if (epi_mode == kEpiNhwc && epi.residual && mode == kModeGeneral && g.O % 4 == 0 && reinterpret_cast<uintptr_t>(epi.residual) % 16 == 0 &&
         load_driver() == TSB_OK) {
         cuuint64_t dims[2] = {(cuuint64_t)g.O, (cuuint64_t)kp.M_total};
         cuuint64_t strides[1] = {(cuuint64_t)g.O * 4};
@@ -582,33 +582,33 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
         if (epi.out_f32) ok_maps = ok_maps && encode(&map_of, epi.out_f32, true, (uint64_t)r.O);
         if (epi.out_i8) ok_maps = ok_maps && encode(&map_oi, epi.out_i8, false, (uint64_t)epi.out_cp);
         if (ok_maps) {
-            kp.epi_mode = kEpiStaged;
+            epi_mode = kEpiStaged;
             kp.res_prefetch = 0;
             kp.stg_f32 = cfg.staging == 2 ? 1 : 0;
         }
     }
     if (dual) {
-        if (!dual_concat && kp.epi_mode != kEpiStaged) return fail(TSB_ERR_UNSUPPORTED, "projected shortcut: the output tensor maps could not be encoded");
-        if (dual_concat && kp.epi_mode != kEpiStaged && kp.epi_mode != kEpiI8Nhwc && kp.epi_mode != kEpiNhwc)
-            return fail(TSB_ERR_UNSUPPORTED, "concatenated input: outputs must be pixel-major fp32 and / or NHWC_PAD int8 with half-away rounding");
+        if (!dual_concat && epi_mode != kEpiStaged) return fail(TSB_ERR_UNSUPPORTED, "projected shortcut: the output tensor maps could not be encoded");
+        if (dual_concat && epi_mode != kEpiStaged && epi_mode != kEpiI8Nhwc)
+            return fail(TSB_ERR_UNSUPPORTED, "concatenated input: outputs must be pixel-major fp32 and / or NHWC_PAD int8");
         const ConvGeom &s = dual->view->g;
         DualParams dp;
         dp.map_a2 = dual->map_a; dp.map_b2 = dual->map_b;
         dp.dq2 = dual->dq; dp.bias2 = dual->bias;
         dp.concat = dual->dq == nullptr ? 1 : 0;
         dp.k2_iters = s.Cp / cfg.bk; dp.Cp2 = s.Cp; dp.a2_tiled = dual->view->a_tiled; dp.sh2 = s.sh; dp.sw2 = s.sw;
-        if (cfg.bn == 256 && cfg.bk == 64) return launch<256, 64, false, kModeGeneral, true>(cfg, map_a, map_b, map_r, map_of, map_oi, kp, epi, stream, dp);
-        if (cfg.bn == 256 && cfg.bk == 128) return launch<256, 128, false, kModeGeneral, true>(cfg, map_a, map_b, map_r, map_of, map_oi, kp, epi, stream, dp);
-        if (cfg.bn == 128 && cfg.bk == 64) return launch<128, 64, false, kModeGeneral, true>(cfg, map_a, map_b, map_r, map_of, map_oi, kp, epi, stream, dp);
-        if (cfg.bn == 128 && cfg.bk == 128) return launch<128, 128, false, kModeGeneral, true>(cfg, map_a, map_b, map_r, map_of, map_oi, kp, epi, stream, dp);
-        if (cfg.bn == 64 && cfg.bk == 64 && dual_concat) return launch<64, 64, false, kModeGeneral, true>(cfg, map_a, map_b, map_r, map_of, map_oi, kp, epi, stream, dp);
-        if (cfg.bn == 64 && cfg.bk == 128 && dual_concat) return launch<64, 128, false, kModeGeneral, true>(cfg, map_a, map_b, map_r, map_of, map_oi, kp, epi, stream, dp);
+#define TSB_TC_CASE(BN_, BK_, SWAP_, MODE_, EPI_, DUAL_)                                                                     \
+    if constexpr (DUAL_)                                                                                                     \
+        if (cfg.bn == BN_ && cfg.bk == BK_ && epi_mode == EPI_ && (BN_ > 64 || dual_concat))                                 \
+            return launch<BN_, BK_, SWAP_, MODE_, EPI_, true>(cfg, map_a, map_b, map_r, map_of, map_oi, kp, epi, stream, dp);
+        TSB_TC_PART_9(TSB_TC_CASE)
+#undef TSB_TC_CASE
         return fail(TSB_ERR_UNSUPPORTED, "no projected-shortcut kernel for tile %dx%d", cfg.bn, cfg.bk);
     }
-#define TSB_TC_CASE(BN_, BK_, SWAP_, MODE_, DUAL_)                                                                           \
+#define TSB_TC_CASE(BN_, BK_, SWAP_, MODE_, EPI_, DUAL_)                                                                           \
     if constexpr (!DUAL_)                                                                                                    \
-        if (cfg.bn == BN_ && cfg.bk == BK_ && (cfg.swap != 0) == SWAP_ && mode == MODE_)                                     \
-            return launch<BN_, BK_, SWAP_, MODE_, false>(cfg, map_a, map_b, map_r, map_of, map_oi, kp, epi, stream, NoDual());
+        if (cfg.bn == BN_ && cfg.bk == BK_ && (cfg.swap != 0) == SWAP_ && mode == MODE_ && epi_mode == EPI_)                 \
+            return launch<BN_, BK_, SWAP_, MODE_, EPI_, false>(cfg, map_a, map_b, map_r, map_of, map_oi, kp, epi, stream, NoDual());
     TSB_TC_ALL(TSB_TC_CASE)
 #undef TSB_TC_CASE
     return fail(TSB_ERR_UNSUPPORTED, "no tcgen05 kernel for tile %dx%d", cfg.bn, cfg.bk);

@@ -1,11 +1,11 @@
-// One group of instances of the tensor-core kernel: compiled once per group with -DTSB_TC_PART=0..7.
+// One group of instances of the tensor-core kernel: compiled once per group with -DTSB_TC_PART=0..9.
 #include "conv_tc_kernel.cuh"
 
 namespace tsb {
 namespace tc {
 
-#define TSB_TC_INSTANCE(BN_, BK_, SWAP_, MODE_, DUAL_)                                                                      \
-    template int launch<BN_, BK_, SWAP_, MODE_, DUAL_>(const Config &, const CUtensorMap &, const CUtensorMap &,            \
+#define TSB_TC_INSTANCE(BN_, BK_, SWAP_, MODE_, EPI_, DUAL_)                                                                      \
+    template int launch<BN_, BK_, SWAP_, MODE_, EPI_, DUAL_>(const Config &, const CUtensorMap &, const CUtensorMap &,            \
                                                        const CUtensorMap &, const CUtensorMap &, const CUtensorMap &,       \
                                                        const KernelParams &, const EpiParams &, cudaStream_t,               \
                                                        const std::conditional_t<DUAL_, DualParams, NoDual> &);

@@ -251,19 +251,24 @@ __device__ __forceinline__ constexpr uint32_t instr_desc() {
 // ---------------------------------------------------------------------------------------------------------
 // epilogue: 32 accumulator columns of one output pixel (one thread) at a time
 // ---------------------------------------------------------------------------------------------------------
+// Which one a launch takes is a template parameter of the kernel (EPI): an instance holds the code of one class only.  With all
+// classes in one kernel every class paid for the others: 700 bytes of spills in all of them (now none, 340 in the staged class),
+// and a variant more cost the layers that never ran it 3-8 %.  Measured with the classes apart: the five sweep layers at batch 32
+// 126 -> 115 us, a ResNet-50 pass of 64 images 1.42 -> 1.35 ms.
 constexpr int kEpiGeneric = 0;   // any combination of outputs, element by element
 constexpr int kEpiF32Nchw = 1;   // fp32 NCHW output only (the operator's own output)
 constexpr int kEpiI8Nhwc = 2;    // requantized int8 NHWC_PAD output only, half-away rounding, one scale per sample
-constexpr int kEpiNhwc = 3;      // fp32 [N][P][O] residual in and/or fp32 [N][P][O] out and/or int8 NHWC_PAD out (normal orientation)
+constexpr int kEpiNhwc = 3;      // fp32 [N][P][O] residual in and/or fp32 [N][P][O] out and/or int8 NHWC_PAD out (swapped orientation)
 constexpr int kEpiStaged = 4;    // the same outputs through shared-memory tiles and tensor-map loads / stores (normal orientation)
 constexpr uint32_t kStageF32Bytes = kBM * 32 * 4;   // one staged fp32 tile: 128 pixels x 32 channels, 128-byte rows, swizzle 128B
 constexpr uint32_t kStageI8Bytes = kBM * 32;        // one staged int8 tile: 128 pixels x 32 channels, 32-byte rows
 constexpr int kQuads = 4;                           // the sixteen epilogue warps form four quads of one warp per lane quarter
 
-template <int ACT, bool HAS_BIAS>
+// (a layer without a bias adds a zero: the same value up to the sign of a zero, which the operators' results are compared up
+// to anyway)
+template <int ACT>
 __device__ __forceinline__ float epi_value(int acc, float dq, float bias, float leaky) {
-    float f = __fmul_rn(__int2float_rn(acc), dq);
-    if (HAS_BIAS) f = __fadd_rn(f, bias);
+    float f = __fadd_rn(__fmul_rn(__int2float_rn(acc), dq), bias);
     if (ACT == TSB_ACT_RELU) f = fmaxf(f, 0.0f);   // finite values only: same result as x > 0 ? x : 0
     if (ACT == TSB_ACT_LEAKY_RELU) f = f > 0.0f ? f : __fmul_rn(f, leaky);
     return f;
@@ -276,6 +281,29 @@ __device__ __forceinline__ int half_away_s32(float t) {
     const float mag = __fadd_rz(fabsf(t), 0.5f);
     const float signed_mag = __int_as_float((__float_as_int(mag) & 0x7fffffff) | (__float_as_int(t) & 0x80000000));
     return __float2int_rz(signed_mag);
+}
+
+// The rounding of a requantize, as a signed 32-bit integer: half-to-even where one scale covers the tensor (a batch of one;
+// the last count % 8 elements excepted, see fix_tail), half away from zero otherwise.  A compile-time choice: one conversion
+// per value either way.  (Element by element, as single-scale outputs once went, a 128 x 64 tile took 15 us where this takes 2: a
+// CSPDarknet53-shaped pass of one 608 x 608 image 2.65 -> 0.61 ms.)
+template <bool EVEN>
+__device__ __forceinline__ int round_s32(float t) {
+    if (EVEN) return __float2int_rn(t);
+    return half_away_s32(t);
+}
+// ... and as a saturated int8
+template <bool EVEN>
+__device__ __forceinline__ int round_s8(float t) {
+    int q;
+    if (EVEN) {
+        asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(q) : "f"(t));
+    } else {
+        const float mag = __fadd_rz(fabsf(t), 0.5f);
+        const float sm = __int_as_float((__float_as_int(mag) & 0x7fffffff) | (__float_as_int(t) & 0x80000000));
+        asm("cvt.rzi.sat.s8.f32 %0, %1;" : "=r"(q) : "f"(sm));
+    }
+    return q;
 }
 
 // four signed integers -> four int8 with saturation to [-128,127], v0 in the lowest byte
@@ -301,42 +329,47 @@ __device__ __forceinline__ float max3_nan(float a, float b, float c) {
 }
 
 // ---- fast paths, normal orientation: the thread owns one PIXEL (its tensor-memory lane) and 32 consecutive channels
-template <int ACT, bool HAS_BIAS, int W>
+template <int ACT, int W>
 __device__ __forceinline__ void store_f32_nchw_t(const int (&v)[W], const float *__restrict__ dq,
                                                  const float *__restrict__ bias, float leaky, float *__restrict__ dst,
-                                                 uint32_t stride) {
+                                                 uint32_t stride, int channels) {
+    if (channels < W) {    // the last chunk of a channel count that is no multiple of 32
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+            if (j < channels) dst[(uint32_t)j * stride] = epi_value<ACT>(v[j], dq[j], bias[j], leaky);
+        return;
+    }
 #pragma unroll
     for (int j4 = 0; j4 < W / 4; ++j4) {
         const float4 d4 = *reinterpret_cast<const float4 *>(dq + 4 * j4);
         const float4 b4 = *reinterpret_cast<const float4 *>(bias + 4 * j4);
-        dst[(uint32_t)(4 * j4 + 0) * stride] = epi_value<ACT, HAS_BIAS>(v[4 * j4 + 0], d4.x, b4.x, leaky);
-        dst[(uint32_t)(4 * j4 + 1) * stride] = epi_value<ACT, HAS_BIAS>(v[4 * j4 + 1], d4.y, b4.y, leaky);
-        dst[(uint32_t)(4 * j4 + 2) * stride] = epi_value<ACT, HAS_BIAS>(v[4 * j4 + 2], d4.z, b4.z, leaky);
-        dst[(uint32_t)(4 * j4 + 3) * stride] = epi_value<ACT, HAS_BIAS>(v[4 * j4 + 3], d4.w, b4.w, leaky);
+        dst[(uint32_t)(4 * j4 + 0) * stride] = epi_value<ACT>(v[4 * j4 + 0], d4.x, b4.x, leaky);
+        dst[(uint32_t)(4 * j4 + 1) * stride] = epi_value<ACT>(v[4 * j4 + 1], d4.y, b4.y, leaky);
+        dst[(uint32_t)(4 * j4 + 2) * stride] = epi_value<ACT>(v[4 * j4 + 2], d4.z, b4.z, leaky);
+        dst[(uint32_t)(4 * j4 + 3) * stride] = epi_value<ACT>(v[4 * j4 + 3], d4.w, b4.w, leaky);
     }
 }
 
 // The same with an fp32 NCHW residual (operator "add" between add_bias and the activation, or after the activation): the
 // residual is read where the result is written, so a warp's 32 pixels make one coalesced line per channel either way.
-template <int ACT, bool HAS_BIAS, int W, bool AFTER>
+template <int ACT, int W, bool AFTER>
 __device__ __forceinline__ void store_f32_nchw_res_t(const int (&v)[W], const float *__restrict__ dq,
                                                      const float *__restrict__ bias, float leaky, const float *__restrict__ res,
-                                                     float *__restrict__ dst, uint32_t stride) {
+                                                     float *__restrict__ dst, uint32_t stride, int channels) {
 #pragma unroll
     for (int j8 = 0; j8 < W / 8; ++j8) {
         float r[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) r[k] = __ldg(res + (uint32_t)(8 * j8 + k) * stride);
+        for (int k = 0; k < 8; ++k) r[k] = 8 * j8 + k < channels ? __ldg(res + (uint32_t)(8 * j8 + k) * stride) : 0.0f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int j = 8 * j8 + k;
-            float t = __fmul_rn(__int2float_rn(v[j]), dq[j]);
-            if (HAS_BIAS) t = __fadd_rn(t, bias[j]);
+            float t = __fadd_rn(__fmul_rn(__int2float_rn(v[j]), dq[j]), bias[j]);
             if (!AFTER) t = __fadd_rn(t, r[k]);
             if (ACT == TSB_ACT_RELU) t = fmaxf(t, 0.0f);
             if (ACT == TSB_ACT_LEAKY_RELU) t = t > 0.0f ? t : __fmul_rn(t, leaky);
             if (AFTER) t = __fadd_rn(t, r[k]);
-            dst[(uint32_t)j * stride] = t;
+            if (j < channels) dst[(uint32_t)j * stride] = t;
         }
     }
 }
@@ -344,76 +377,38 @@ __device__ __forceinline__ void store_f32_nchw_res_t(const int (&v)[W], const fl
 // Requantized int8 output.  Returns false when a scaled value was NaN or beyond the int32 range -- those quantize to
 // -128 in the reference (x86 integer-indefinite), which the saturating fast path does not reproduce; the caller
 // then redoes the chunk element by element.
-template <int ACT, bool HAS_BIAS, int W>
+// (columns at or beyond O have zero weights, scale and bias, so they come out as the zeros that the layout's padding channels
+// hold; `bytes` says how much of the chunk lies inside the padded row)
+template <int ACT, bool EVEN, int W>
 __device__ __forceinline__ bool store_i8_nhwc_t(const int (&v)[W], const float *__restrict__ dq,
                                                 const float *__restrict__ bias, float leaky, float rs,
-                                                int8_t *__restrict__ dst) {
+                                                int8_t *__restrict__ dst, int bytes) {
     uint32_t q[W / 4];
     float worst = 0.0f;
 #pragma unroll
     for (int j4 = 0; j4 < W / 4; ++j4) {
         const float4 d4 = *reinterpret_cast<const float4 *>(dq + 4 * j4);
         const float4 b4 = *reinterpret_cast<const float4 *>(bias + 4 * j4);
-        const float t0 = __fmul_rn(epi_value<ACT, HAS_BIAS>(v[4 * j4 + 0], d4.x, b4.x, leaky), rs);
-        const float t1 = __fmul_rn(epi_value<ACT, HAS_BIAS>(v[4 * j4 + 1], d4.y, b4.y, leaky), rs);
-        const float t2 = __fmul_rn(epi_value<ACT, HAS_BIAS>(v[4 * j4 + 2], d4.z, b4.z, leaky), rs);
-        const float t3 = __fmul_rn(epi_value<ACT, HAS_BIAS>(v[4 * j4 + 3], d4.w, b4.w, leaky), rs);
+        const float t0 = __fmul_rn(epi_value<ACT>(v[4 * j4 + 0], d4.x, b4.x, leaky), rs);
+        const float t1 = __fmul_rn(epi_value<ACT>(v[4 * j4 + 1], d4.y, b4.y, leaky), rs);
+        const float t2 = __fmul_rn(epi_value<ACT>(v[4 * j4 + 2], d4.z, b4.z, leaky), rs);
+        const float t3 = __fmul_rn(epi_value<ACT>(v[4 * j4 + 3], d4.w, b4.w, leaky), rs);
         worst = max3_nan(max3_nan(worst, fabsf(t0), fabsf(t1)), fabsf(t2), fabsf(t3));
-        q[j4] = pack_sat_s8(half_away_s32(t0), half_away_s32(t1), half_away_s32(t2), half_away_s32(t3));
+        q[j4] = pack_sat_s8(round_s32<EVEN>(t0), round_s32<EVEN>(t1), round_s32<EVEN>(t2), round_s32<EVEN>(t3));
     }
     if (!(worst < 2147483648.0f)) return false;
 #pragma unroll
-    for (int h = 0; h < W / 16; ++h) *reinterpret_cast<int4 *>(dst + 16 * h) = make_int4(q[4 * h], q[4 * h + 1], q[4 * h + 2], q[4 * h + 3]);
+    for (int h = 0; h < W / 16; ++h)
+        if (16 * h < bytes) *reinterpret_cast<int4 *>(dst + 16 * h) = make_int4(q[4 * h], q[4 * h + 1], q[4 * h + 2], q[4 * h + 3]);
     return true;
 }
 
 // Block-output epilogue of a residual network: v = act(dq*acc + bias + residual); fp32 copy for the next residual and
-// int8 copy for the next convolution.  Each pointer may be null.  All three tensors are pixel-major, so the thread's 32
-// channels are contiguous: 16-byte loads and stores.
-template <int ACT, bool HAS_BIAS, int W, bool AFTER>
-__device__ __forceinline__ bool store_nhwc_t(const int (&v)[W], const float *__restrict__ dq, const float *__restrict__ bias,
-                                             float leaky, const float *__restrict__ res, float *__restrict__ out_f32,
-                                             int8_t *__restrict__ out_i8, float rs) {
-    uint32_t q[W / 4];
-    float worst = 0.0f;
-#pragma unroll
-    for (int j4 = 0; j4 < W / 4; ++j4) {
-        const float4 d4 = *reinterpret_cast<const float4 *>(dq + 4 * j4);
-        const float4 b4 = *reinterpret_cast<const float4 *>(bias + 4 * j4);
-        float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (res) r4 = __ldg(reinterpret_cast<const float4 *>(res) + j4);
-        float f[4];
-        const float dd[4] = {d4.x, d4.y, d4.z, d4.w}, bb[4] = {b4.x, b4.y, b4.z, b4.w}, rr[4] = {r4.x, r4.y, r4.z, r4.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            float t = __fmul_rn(__int2float_rn(v[4 * j4 + k]), dd[k]);
-            if (HAS_BIAS) t = __fadd_rn(t, bb[k]);
-            if (res && !AFTER) t = __fadd_rn(t, rr[k]);
-            if (ACT == TSB_ACT_RELU) t = fmaxf(t, 0.0f);
-            if (ACT == TSB_ACT_LEAKY_RELU) t = t > 0.0f ? t : __fmul_rn(t, leaky);
-            if (res && AFTER) t = __fadd_rn(t, rr[k]);
-            f[k] = t;
-        }
-        if (out_f32) reinterpret_cast<float4 *>(out_f32)[j4] = make_float4(f[0], f[1], f[2], f[3]);
-        if (out_i8) {
-            const float t0 = __fmul_rn(f[0], rs), t1 = __fmul_rn(f[1], rs), t2 = __fmul_rn(f[2], rs), t3 = __fmul_rn(f[3], rs);
-            worst = max3_nan(max3_nan(worst, fabsf(t0), fabsf(t1)), fabsf(t2), fabsf(t3));
-            q[j4] = pack_sat_s8(half_away_s32(t0), half_away_s32(t1), half_away_s32(t2), half_away_s32(t3));
-        }
-    }
-    if (out_i8) {
-        if (!(worst < 2147483648.0f)) return false;
-#pragma unroll
-        for (int h = 0; h < W / 16; ++h) *reinterpret_cast<int4 *>(out_i8 + 16 * h) = make_int4(q[4 * h], q[4 * h + 1], q[4 * h + 2], q[4 * h + 3]);
-    }
-    return true;
-}
-
-// Staged form of the same block epilogue: the thread's 32 channels of residual come from its row of a shared-memory tile
+// int8 copy for the next convolution, each optional.  The thread's 32 channels of residual come from its row of a shared-memory tile
 // that a tensor-map load filled (128-byte rows, 128B swizzle: 16-byte chunk i of row r sits at chunk i ^ (r & 7)), the
 // fp32 results go back into the same places and the int8 results into the thread's 32-byte row of a second tile; tensor-
 // map stores carry both tiles to global memory.  No global address arithmetic, every shared-memory access 16 bytes wide.
-template <int ACT, bool HAS_BIAS, bool AFTER>
+template <int ACT, bool EVEN, bool AFTER>
 __device__ __forceinline__ bool staged_chunk_t(const int (&v)[32], const float *__restrict__ dq, const float *__restrict__ bias,
                                                float leaky, float4 *__restrict__ r_row, int key, bool has_res, bool has_f32,
                                                int4 *__restrict__ q_row, bool has_i8, float rs) {
@@ -429,8 +424,7 @@ __device__ __forceinline__ bool staged_chunk_t(const int (&v)[32], const float *
         const float dd[4] = {d4.x, d4.y, d4.z, d4.w}, bb[4] = {b4.x, b4.y, b4.z, b4.w}, rr[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            float t = __fmul_rn(__int2float_rn(v[4 * j4 + k]), dd[k]);
-            if (HAS_BIAS) t = __fadd_rn(t, bb[k]);
+            float t = __fadd_rn(__fmul_rn(__int2float_rn(v[4 * j4 + k]), dd[k]), bb[k]);
             // without a residual rr is zero: adding it changes nothing but the sign of a negative zero, which the
             // operators' results are compared up to anyway (relu and leaky_relu do not pin it either)
             if (!AFTER) t = __fadd_rn(t, rr[k]);
@@ -443,7 +437,7 @@ __device__ __forceinline__ bool staged_chunk_t(const int (&v)[32], const float *
         if (has_i8) {
             const float t0 = __fmul_rn(f[0], rs), t1 = __fmul_rn(f[1], rs), t2 = __fmul_rn(f[2], rs), t3 = __fmul_rn(f[3], rs);
             worst = max3_nan(max3_nan(worst, fabsf(t0), fabsf(t1)), fabsf(t2), fabsf(t3));
-            q[j4] = pack_sat_s8(half_away_s32(t0), half_away_s32(t1), half_away_s32(t2), half_away_s32(t3));
+            q[j4] = pack_sat_s8(round_s32<EVEN>(t0), round_s32<EVEN>(t1), round_s32<EVEN>(t2), round_s32<EVEN>(t3));
         }
     }
     if (has_i8) {
@@ -456,53 +450,62 @@ __device__ __forceinline__ bool staged_chunk_t(const int (&v)[32], const float *
 
 // ---- fast paths, swapped orientation: the thread owns one CHANNEL (its lane) and 32 consecutive pixels; dq and bias
 // are per-thread scalars
-template <int ACT, bool HAS_BIAS>
+template <int ACT>
 __device__ __forceinline__ void swap_f32_run(const int (&v)[32], float dq, float bias, float leaky, float *__restrict__ dst) {
     // 32 consecutive pixels of one channel plane: 128 contiguous bytes
     if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
 #pragma unroll
         for (int j4 = 0; j4 < 8; ++j4) {
             float4 o;
-            o.x = epi_value<ACT, HAS_BIAS>(v[4 * j4 + 0], dq, bias, leaky);
-            o.y = epi_value<ACT, HAS_BIAS>(v[4 * j4 + 1], dq, bias, leaky);
-            o.z = epi_value<ACT, HAS_BIAS>(v[4 * j4 + 2], dq, bias, leaky);
-            o.w = epi_value<ACT, HAS_BIAS>(v[4 * j4 + 3], dq, bias, leaky);
+            o.x = epi_value<ACT>(v[4 * j4 + 0], dq, bias, leaky);
+            o.y = epi_value<ACT>(v[4 * j4 + 1], dq, bias, leaky);
+            o.z = epi_value<ACT>(v[4 * j4 + 2], dq, bias, leaky);
+            o.w = epi_value<ACT>(v[4 * j4 + 3], dq, bias, leaky);
             reinterpret_cast<float4 *>(dst)[j4] = o;
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) dst[j] = epi_value<ACT, HAS_BIAS>(v[j], dq, bias, leaky);
+        for (int j = 0; j < 32; ++j) dst[j] = epi_value<ACT>(v[j], dq, bias, leaky);
     }
+}
+
+// The same where the chunk ends the tensor (npix < 32) or crosses an image boundary: pixels from `split` on belong to the next
+// image, `jump` floats further on.  For images of at least 32 pixels (one boundary at most).
+template <int ACT>
+__device__ __forceinline__ void swap_f32_split_run(const int (&v)[32], float dq, float bias, float leaky, float *__restrict__ dst,
+                                                   int npix, int split, uint32_t jump) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+        if (j < npix) dst[(uint32_t)j + (j >= split ? jump : 0u)] = epi_value<ACT>(v[j], dq, bias, leaky);
 }
 
 // int8 NHWC_PAD output: for one pixel the 32 lanes of the warp hold 32 consecutive channels, so each byte store
 // instruction of the warp writes one full 32-byte sector.  The first `split` pixels use rs0, the rest rs1 (the chunk
 // crosses at most one image boundary).
 // Returns false if a value needs the slow path (NaN / beyond int32); the decision is uniform over the warp.
-template <int ACT, bool HAS_BIAS>
+template <int ACT, bool EVEN>
 __device__ __forceinline__ bool swap_i8_run(const int (&v)[32], float dq, float bias, float leaky, float rs0, float rs1,
-                                            int split, bool write, int8_t *__restrict__ dst, uint32_t pixel_stride) {
+                                            int split, bool write, int8_t *__restrict__ dst, uint32_t pixel_stride, int npix) {
     float worst = 0.0f;
     int q[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
-        const float t = __fmul_rn(epi_value<ACT, HAS_BIAS>(v[j], dq, bias, leaky), j < split ? rs0 : rs1);
+        const float t = __fmul_rn(epi_value<ACT>(v[j], dq, bias, leaky), j < split ? rs0 : rs1);
         worst = max_nan(worst, fabsf(t));
-        const float mag = __fadd_rz(fabsf(t), 0.5f);
-        const float sm = __int_as_float((__float_as_int(mag) & 0x7fffffff) | (__float_as_int(t) & 0x80000000));
-        asm("cvt.rzi.s8.f32 %0, %1;" : "=r"(q[j]) : "f"(sm));  // float -> int8 conversions saturate
+        q[j] = round_s8<EVEN>(t);
     }
     if (__any_sync(0xffffffffu, !(worst < 2147483648.0f))) return false;
     if (write) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) dst[(uint32_t)j * pixel_stride] = (int8_t)q[j];
+        for (int j = 0; j < 32; ++j)
+            if (j < npix) dst[(uint32_t)j * pixel_stride] = (int8_t)q[j];
     }
     return true;
 }
 
 // Patch mode, swapped orientation: the 32 accumulators of a chunk are 4 tile rows of 8 pixels of one channel.
 // rows_live / cols_live say how much of that 4 x 8 block lies inside the image (uniform over the warp).
-template <int ACT, bool HAS_BIAS>
+template <int ACT, bool EVEN>
 __device__ __forceinline__ bool patch_i8_run(const int (&v)[32], float dq, float bias, float leaky, float rs, bool write,
                                              int8_t *__restrict__ dst, uint32_t pixel_stride, uint32_t row_stride,
                                              int rows_live, int cols_live) {
@@ -510,12 +513,10 @@ __device__ __forceinline__ bool patch_i8_run(const int (&v)[32], float dq, float
     int q[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
-        const float t = __fmul_rn(epi_value<ACT, HAS_BIAS>(v[j], dq, bias, leaky), rs);
+        const float t = __fmul_rn(epi_value<ACT>(v[j], dq, bias, leaky), rs);
         const bool live = (j >> 3) < rows_live && (j & 7) < cols_live;
         worst = max_nan(worst, live ? fabsf(t) : 0.0f);
-        const float mag = __fadd_rz(fabsf(t), 0.5f);
-        const float sm = __int_as_float((__float_as_int(mag) & 0x7fffffff) | (__float_as_int(t) & 0x80000000));
-        asm("cvt.rzi.s8.f32 %0, %1;" : "=r"(q[j]) : "f"(sm));
+        q[j] = round_s8<EVEN>(t);
     }
     if (__any_sync(0xffffffffu, !(worst < 2147483648.0f))) return false;
     if (write) {
@@ -525,7 +526,7 @@ __device__ __forceinline__ bool patch_i8_run(const int (&v)[32], float dq, float
     }
     return true;
 }
-template <int ACT, bool HAS_BIAS>
+template <int ACT>
 __device__ __forceinline__ void patch_f32_run(const int (&v)[32], float dq, float bias, float leaky, float *__restrict__ dst,
                                               uint32_t row_stride, int rows_live, int cols_live) {
     // fp32 NCHW: each tile row is 8 consecutive floats of one channel plane
@@ -538,23 +539,23 @@ __device__ __forceinline__ void patch_f32_run(const int (&v)[32], float dq, floa
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 float4 o;
-                o.x = epi_value<ACT, HAS_BIAS>(v[8 * r + 4 * h + 0], dq, bias, leaky);
-                o.y = epi_value<ACT, HAS_BIAS>(v[8 * r + 4 * h + 1], dq, bias, leaky);
-                o.z = epi_value<ACT, HAS_BIAS>(v[8 * r + 4 * h + 2], dq, bias, leaky);
-                o.w = epi_value<ACT, HAS_BIAS>(v[8 * r + 4 * h + 3], dq, bias, leaky);
+                o.x = epi_value<ACT>(v[8 * r + 4 * h + 0], dq, bias, leaky);
+                o.y = epi_value<ACT>(v[8 * r + 4 * h + 1], dq, bias, leaky);
+                o.z = epi_value<ACT>(v[8 * r + 4 * h + 2], dq, bias, leaky);
+                o.w = epi_value<ACT>(v[8 * r + 4 * h + 3], dq, bias, leaky);
                 reinterpret_cast<float4 *>(row)[h] = o;
             }
         } else {
 #pragma unroll
             for (int cidx = 0; cidx < 8; ++cidx)
-                if (cidx < cols_live) row[cidx] = epi_value<ACT, HAS_BIAS>(v[8 * r + cidx], dq, bias, leaky);
+                if (cidx < cols_live) row[cidx] = epi_value<ACT>(v[8 * r + cidx], dq, bias, leaky);
         }
     }
 }
 
 // Pixel-major fp32 tensors in the swapped orientation: for one pixel the warp's 32 lanes touch 32 consecutive floats
 // (residual read, fp32 write) and 32 consecutive int8 (requantized write): every access is one coalesced line.
-template <int ACT, bool HAS_BIAS, bool AFTER>
+template <int ACT, bool EVEN, bool AFTER>
 __device__ __forceinline__ bool swap_nhwc_run(const int (&v)[32], float dq, float bias, float leaky,
                                               const float *__restrict__ res, float *__restrict__ out_f32,
                                               int8_t *__restrict__ out_i8, bool write_i8, float rs0, float rs1, int split,
@@ -568,8 +569,7 @@ __device__ __forceinline__ bool swap_nhwc_run(const int (&v)[32], float dq, floa
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int j = j0 + k;
-            float t = __fmul_rn(__int2float_rn(v[j]), dq);
-            if (HAS_BIAS) t = __fadd_rn(t, bias);
+            float t = __fadd_rn(__fmul_rn(__int2float_rn(v[j]), dq), bias);
             if (res && !AFTER) t = __fadd_rn(t, r[k]);
             if (ACT == TSB_ACT_RELU) t = fmaxf(t, 0.0f);
             if (ACT == TSB_ACT_LEAKY_RELU) t = t > 0.0f ? t : __fmul_rn(t, leaky);
@@ -578,10 +578,7 @@ __device__ __forceinline__ bool swap_nhwc_run(const int (&v)[32], float dq, floa
             if (out_i8) {
                 const float u = __fmul_rn(t, j < split ? rs0 : rs1);
                 worst = max_nan(worst, fabsf(u));
-                const float mag = __fadd_rz(fabsf(u), 0.5f);
-                const float sm = __int_as_float((__float_as_int(mag) & 0x7fffffff) | (__float_as_int(u) & 0x80000000));
-                int q;
-                asm("cvt.rzi.s8.f32 %0, %1;" : "=r"(q) : "f"(sm));
+                const int q = round_s8<EVEN>(u);
                 if (write_i8) out_i8[(uint32_t)j * out_cp] = (int8_t)q;   // redone by the caller if the check below fails
             }
         }
@@ -589,43 +586,25 @@ __device__ __forceinline__ bool swap_nhwc_run(const int (&v)[32], float dq, floa
     return !__any_sync(0xffffffffu, !(worst < 2147483648.0f));
 }
 
-// run FN<activation, has_bias>(args...) for the runtime activation / bias combination
-#define TSB_EPI_DISPATCH_W(RESULT, FN, W_, ...)                                                           \
-    do {                                                                                                  \
-        if (has_bias) {                                                                                   \
-            if (act == TSB_ACT_RELU) RESULT FN<TSB_ACT_RELU, true, W_>(__VA_ARGS__);                      \
-            else if (act == TSB_ACT_LEAKY_RELU) RESULT FN<TSB_ACT_LEAKY_RELU, true, W_>(__VA_ARGS__);     \
-            else RESULT FN<TSB_ACT_NONE, true, W_>(__VA_ARGS__);                                          \
-        } else {                                                                                          \
-            if (act == TSB_ACT_RELU) RESULT FN<TSB_ACT_RELU, false, W_>(__VA_ARGS__);                     \
-            else if (act == TSB_ACT_LEAKY_RELU) RESULT FN<TSB_ACT_LEAKY_RELU, false, W_>(__VA_ARGS__);    \
-            else RESULT FN<TSB_ACT_NONE, false, W_>(__VA_ARGS__);                                         \
-        }                                                                                                 \
-    } while (0)
-// the two residual epilogues: a second instantiation for "residual after the activation"
-#define TSB_EPI_DISPATCH_RES_W(RESULT, FN, W_, ...)                                                       \
-    do {                                                                                                  \
-        if (epi.res_after) TSB_EPI_DISPATCH_W(RESULT, FN, W_ TSB_COMMA true, __VA_ARGS__);                \
-        else TSB_EPI_DISPATCH_W(RESULT, FN, W_ TSB_COMMA false, __VA_ARGS__);                             \
-    } while (0)
-#define TSB_COMMA ,
-#define TSB_EPI_DISPATCH_SWAPRES(RESULT, FN, ...)                                                         \
-    do {                                                                                                  \
-        if (epi.res_after) TSB_EPI_DISPATCH_W(RESULT, FN, true, __VA_ARGS__);                             \
-        else TSB_EPI_DISPATCH_W(RESULT, FN, false, __VA_ARGS__);                                          \
-    } while (0)
-#define TSB_EPI_DISPATCH(RESULT, FN, ...)                                                                 \
-    do {                                                                                                  \
-        if (has_bias) {                                                                                   \
-            if (act == TSB_ACT_RELU) RESULT FN<TSB_ACT_RELU, true>(__VA_ARGS__);                          \
-            else if (act == TSB_ACT_LEAKY_RELU) RESULT FN<TSB_ACT_LEAKY_RELU, true>(__VA_ARGS__);         \
-            else RESULT FN<TSB_ACT_NONE, true>(__VA_ARGS__);                                              \
-        } else {                                                                                          \
-            if (act == TSB_ACT_RELU) RESULT FN<TSB_ACT_RELU, false>(__VA_ARGS__);                         \
-            else if (act == TSB_ACT_LEAKY_RELU) RESULT FN<TSB_ACT_LEAKY_RELU, false>(__VA_ARGS__);        \
-            else RESULT FN<TSB_ACT_NONE, false>(__VA_ARGS__);                                             \
-        }                                                                                                 \
-    } while (0)
+// Calls f(activation) / f(activation, half-to-even) / ... with the run-time choices as compile-time constants.
+template <typename F>
+__device__ __forceinline__ void with_act(int act, F f) {
+    if (act == TSB_ACT_RELU) f(std::integral_constant<int, TSB_ACT_RELU>());
+    else if (act == TSB_ACT_LEAKY_RELU) f(std::integral_constant<int, TSB_ACT_LEAKY_RELU>());
+    else f(std::integral_constant<int, TSB_ACT_NONE>());
+}
+template <typename F>
+__device__ __forceinline__ void with_act_flag(int act, int flag, F f) {
+    if (flag) with_act(act, [&](auto a) { f(a, std::true_type()); });
+    else with_act(act, [&](auto a) { f(a, std::false_type()); });
+}
+template <typename F>
+__device__ __forceinline__ void with_act_flags(int act, int flag, int flag2, F f) {
+    if (flag2) with_act_flag(act, flag, [&](auto a, auto e) { f(a, e, std::true_type()); });
+    else with_act_flag(act, flag, [&](auto a, auto e) { f(a, e, std::false_type()); });
+}
+// (the constant behind such an argument)
+#define TSB_VAL(x) decltype(x)::value
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int (&v)[16]) {
     asm volatile(
@@ -643,6 +622,21 @@ __device__ __forceinline__ int tmem_ld1(uint32_t taddr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     return r;
+}
+
+// One scale rounds half to even, except the last count % 8 elements of the tensor (in NCHW order), which round half away from
+// zero (epi.tail says whether there are any).  The fast paths round everything half to even; this redoes, element by element, the few
+// columns of a chunk that hold such an element.  n_of(j), o_of(j), p_of(j): image, channel and pixel of this thread's column j;
+// ok(j): whether the column is one of its outputs.  Called by whole warps.
+template <typename Ok, typename N, typename O, typename P>
+__device__ __forceinline__ void fix_tail(const EpiParams &epi, uint32_t taddr, Ok ok, N n_of, O o_of, P p_of) {
+#pragma unroll 1
+    for (int j = 0; j < 32; ++j) {
+        const bool mine = ok(j) && ((uint32_t)(n_of(j) * epi.O + o_of(j)) * (uint32_t)epi.P + (uint32_t)p_of(j)) >= epi.rne_limit;
+        if (!__any_sync(0xffffffffu, mine)) continue;
+        const int a = tmem_ld1(taddr + (uint32_t)j);
+        if (mine) epilogue_store_one(epi, n_of(j), o_of(j), p_of(j), a);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -674,7 +668,6 @@ struct KernelParams {
     int num_m_tiles, num_n_tiles;   // pixel tiles, channel tiles
     FastDiv d_P, d_OW, d_m_tiles, d_n_tiles, d_segs, d_OH, d_dh;   // dividers by P, OW, num_m_tiles, num_n_tiles, rows_segs, rows_OH, dh
     int per_sample_scale;  // requantize: scale index = image index
-    int epi_mode;          // kEpi*: which epilogue code path full 32-column chunks take
     int a_tiled;           // activations are a plain [M][Cp] matrix (1x1, stride 1, no padding): 2-D tile loads
     // shared-memory plan (bytes from the 1024-aligned base)
     int stages;            // pipeline stages (<= kMaxStages)
@@ -779,7 +772,7 @@ __host__ __device__ constexpr uint32_t num_barriers(int stages) { return 2u * (u
 // instruction where N = O would leave it half or three-quarters empty.
 // MODE: how activations reach shared memory -- kModeGeneral (im2col or plain 2-D tile loads), kModeRows (raw-row), kModePatch.
 // A compile-time parameter: the role loops of each mode stay short and keep their registers.
-template <int BN, int BK, bool SWAP, int MODE, bool DUAL = false>
+template <int BN, int BK, bool SWAP, int MODE, int EPI, bool DUAL>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_of,
@@ -787,6 +780,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                   const __grid_constant__ EpiParams epi,
                   const __grid_constant__ std::conditional_t<DUAL, DualParams, NoDual> dual) {
     static_assert(!DUAL || (!SWAP && MODE == kModeGeneral), "projected-shortcut kernels: normal orientation, general mode");
+    static_assert(SWAP ? EPI != kEpiStaged : EPI != kEpiNhwc, "pixel-major fp32 tensors: staged tiles where a thread owns a pixel");
     constexpr int PIX = SWAP ? BN : kBM;      // pixels per tile
     constexpr int CH = SWAP ? kBM : BN;       // output channels per tile
     constexpr uint32_t kPixBytes = PIX * BK, kWgtBytes = CH * BK;
@@ -1262,7 +1256,6 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const int row = quarter * 32 + lane;     // tensor-memory lane this thread reads
         constexpr int kChunks = BN / 32;
         constexpr int CW = 32;                   // normal orientation: columns a warp takes per step
-        const bool has_bias = epi.bias != nullptr;
         const int act = epi.activation;
         uint32_t stg_phase[1] = {0u};            // staged epilogue: phase of this quad's residual barrier
         int table_n = -1;                        // channel tile this group's scale / bias table holds
@@ -1304,7 +1297,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             if (kp.trace && kp.trace[255] != 0) { tc_fence_before(); mbar_arrive(bar_tempty + 8 * acc); continue; }
 #endif
             const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(slot * BN);
-            if (!SWAP) {
+            if constexpr (!SWAP) {
                 int m = m_tile * PIX + row;
                 bool live = m < kp.M_total;
                 if (MODE == kModeRows) {
@@ -1321,7 +1314,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 }
                 const int img = live ? kp.d_P.div(m) : 0;
                 const int p = live ? m - img * kp.P : 0;
-                if (kp.epi_mode == kEpiStaged) {
+                if constexpr (EPI == kEpiStaged) {
                     // ---- staged epilogue: residual in by tensor-map load, fp32 / int8 tiles out by tensor-map stores.
                     // A quad (the four warps of this group that share `part`, one per lane quarter = the tile's 128
                     // pixels) owns one fp32 tile and one int8 tile in shared memory and works through its 32-channel
@@ -1408,8 +1401,11 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         if (real) tmem_ld_wait();
                         bool fine = true;
                         if (stg_ok) {
-                            if (epi.res_after) TSB_EPI_DISPATCH_W(fine =, staged_chunk_t, true, v, t_dq + col0, t_bias + col0, epi.leaky, r_row, key, real && (has_res || (DUAL && !concat)), has_f32, q_row, has_i8, rs);
-                            else TSB_EPI_DISPATCH_W(fine =, staged_chunk_t, false, v, t_dq + col0, t_bias + col0, epi.leaky, r_row, key, real && (has_res || (DUAL && !concat)), has_f32, q_row, has_i8, rs);
+                            with_act_flags(act, epi.even, epi.res_after, [&](auto a, auto even, auto after) {
+                                fine = staged_chunk_t<TSB_VAL(a), TSB_VAL(even), TSB_VAL(after)>(v, t_dq + col0, t_bias + col0, epi.leaky, r_row, key, real && (has_res || (DUAL && !concat)), has_f32, q_row, has_i8, rs);
+                            });
+                            // the tensor's last count % 8 elements round the other way (fix_tail): the chunk goes element by element
+                            if (epi.tail && real && live && ((uint32_t)(img * epi.O + min(o_base + col0 + 31, epi.O - 1)) * (uint32_t)epi.P + (uint32_t)p) >= epi.rne_limit) fine = false;
                         }
                         fence_async_smem();
                         // all four warps have written their rows; the OR says whether any value needs the exact slow path
@@ -1450,17 +1446,9 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     }
                     if (!stg_ok && !*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 7); }
                 } else {
-                // residual boxes of this thread quad ({32 channels, 128 pixels} each), two chunks ahead of their use
-                const bool prefetcher = kp.res_prefetch && MODE != kModePatch && MODE != kModeRows && quarter == 0 && lane == 0;
-                if (prefetcher) {
-                    if (o_base + part * CW < epi.O) tma_prefetch_l2_2d(&map_r, o_base + part * CW, m_tile * PIX);
-                    if (part + parts < BN / CW && o_base + (part + parts) * CW < epi.O) tma_prefetch_l2_2d(&map_r, o_base + (part + parts) * CW, m_tile * PIX);
-                }
 #pragma unroll 1
                 for (int c = part; c < BN / CW; c += parts) {
                     const int col0 = c * CW;
-                    if (prefetcher && c + 2 * parts < BN / CW && o_base + (c + 2 * parts) * CW < epi.O)
-                        tma_prefetch_l2_2d(&map_r, o_base + (c + 2 * parts) * CW, m_tile * PIX);
                     if (o_base + col0 >= epi.O) {
                         // nothing but channel padding in this step: no accumulators to read, only the zero bytes the
                         // NHWC_PAD layout wants in its padding channels
@@ -1472,36 +1460,37 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         }
                         continue;
                     }
-                    const bool full = o_base + col0 + CW <= epi.O;
+                    const int channels = min(CW, epi.O - (o_base + col0));
                     bool done = false;
-                    if (full && kp.epi_mode != kEpiGeneric) {
+                    if constexpr (EPI == kEpiF32Nchw || EPI == kEpiI8Nhwc) {
                         int v[CW];
                         tmem_ldw(taddr0 + (uint32_t)col0, v);
                         tmem_ld_wait();
-                        if (kp.epi_mode == kEpiF32Nchw) {
+                        if constexpr (EPI == kEpiF32Nchw) {
                             if (live) {
                                 const size_t off = (size_t)(img * epi.O + o_base + col0) * (size_t)epi.P + (size_t)p;
                                 float *dst = epi.out_f32 + off;
-                                if (epi.residual) TSB_EPI_DISPATCH_RES_W(, store_f32_nchw_res_t, CW, v, t_dq + col0, t_bias + col0, epi.leaky, epi.residual + off, dst, (uint32_t)epi.P);
-                                else TSB_EPI_DISPATCH_W(, store_f32_nchw_t, CW, v, t_dq + col0, t_bias + col0, epi.leaky, dst, (uint32_t)epi.P);
+                                if (epi.residual) with_act_flag(act, epi.res_after, [&](auto a, auto after) {
+                                    store_f32_nchw_res_t<TSB_VAL(a), CW, TSB_VAL(after)>(v, t_dq + col0, t_bias + col0, epi.leaky, epi.residual + off, dst, (uint32_t)epi.P, channels);
+                                });
+                                else with_act(act, [&](auto a) {
+                                    store_f32_nchw_t<TSB_VAL(a), CW>(v, t_dq + col0, t_bias + col0, epi.leaky, dst, (uint32_t)epi.P, channels);
+                                });
                             }
                             done = true;
-                        } else if (kp.epi_mode == kEpiI8Nhwc) {
+                        } else {
                             const float rs = epi.nscales == 1 ? epi.rq_scales[0] : epi.rq_scales[img];
                             int8_t *dst = epi.out_i8 + (size_t)m * epi.out_cp + o_base + col0;
                             bool fine = true;
-                            if (live) TSB_EPI_DISPATCH_W(fine =, store_i8_nhwc_t, CW, v, t_dq + col0, t_bias + col0, epi.leaky, rs, dst);
-                            done = !__any_sync(0xffffffffu, !fine);
-                        } else {
-                            const float rs = epi.nscales == 1 ? epi.rq_scales[0] : epi.rq_scales[img];
-                            const size_t f_off = (size_t)m * epi.O + o_base + col0;
-                            const float *res = epi.residual ? epi.residual + f_off : nullptr;
-                            float *of = epi.out_f32 ? epi.out_f32 + f_off : nullptr;
-                            int8_t *oi = epi.out_i8 ? epi.out_i8 + (size_t)m * epi.out_cp + o_base + col0 : nullptr;
-                            bool fine = true;
-                            if (live) TSB_EPI_DISPATCH_RES_W(fine =, store_nhwc_t, CW, v, t_dq + col0, t_bias + col0, epi.leaky, res, of, oi, rs);
+                            if (live) with_act_flag(act, epi.even, [&](auto a, auto even) {
+                                fine = store_i8_nhwc_t<TSB_VAL(a), TSB_VAL(even), CW>(v, t_dq + col0, t_bias + col0, epi.leaky, rs, dst, epi.out_cp - (o_base + col0));
+                            });
                             done = !__any_sync(0xffffffffu, !fine);
                         }
+                        if (EPI == kEpiI8Nhwc && epi.tail && done &&
+                            __any_sync(0xffffffffu, live && ((uint32_t)(img * epi.O + o_base + col0 + channels - 1) * (uint32_t)epi.P + (uint32_t)p) >= epi.rne_limit))
+                            fix_tail(epi, taddr0 + (uint32_t)col0, [&](int j) { return live && j < channels; }, [&](int) { return img; },
+                                     [&](int j) { return o_base + col0 + j; }, [&](int) { return p; });
                     }
                     if (!done) {
                         // element by element: any combination of outputs, residual, partial channel chunks
@@ -1530,7 +1519,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     p_c = p_rem - p_r * kp.patch_tiles_w;
                 }
                 // residual boxes of this thread quad ({128 channels, 32 pixels} each), two chunks ahead of their use
-                const bool prefetcher = kp.res_prefetch && MODE != kModePatch && quarter == 0 && lane == 0;
+                const bool prefetcher = EPI == kEpiNhwc && kp.res_prefetch && MODE != kModePatch && quarter == 0 && lane == 0;
                 if (prefetcher) {
                     if (m_tile * PIX + part * 32 < kp.M_total) tma_prefetch_l2_2d(&map_r, o_base, m_tile * PIX + part * 32);
                     if (part + parts < kChunks && m_tile * PIX + (part + parts) * 32 < kp.M_total) tma_prefetch_l2_2d(&map_r, o_base, m_tile * PIX + (part + parts) * 32);
@@ -1547,21 +1536,27 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         const int rows_live = min(4, kp.OH - oh0), cols_live = min(8, kp.OW - ow0);
                         const int p0 = oh0 * kp.OW + ow0;
                         bool done = false;
-                        if (kp.epi_mode == kEpiF32Nchw || kp.epi_mode == kEpiI8Nhwc) {
+                        if constexpr (EPI == kEpiF32Nchw || EPI == kEpiI8Nhwc) {
                             int v[32];
                             tmem_ld32(taddr0 + (uint32_t)col0, v);
                             tmem_ld_wait();
-                            if (kp.epi_mode == kEpiF32Nchw) {
+                            if constexpr (EPI == kEpiF32Nchw) {
                                 if (ch_live) {
                                     float *dst = epi.out_f32 + ((size_t)(p_img * epi.O + o) * (size_t)epi.P + (size_t)p0);
-                                    TSB_EPI_DISPATCH(, patch_f32_run, v, my_dq, my_bias, epi.leaky, dst, (uint32_t)kp.OW, rows_live, cols_live);
+                                    with_act(act, [&](auto a) { patch_f32_run<TSB_VAL(a)>(v, my_dq, my_bias, epi.leaky, dst, (uint32_t)kp.OW, rows_live, cols_live); });
                                 }
                                 done = true;
                             } else {
                                 const float rs = epi.nscales == 1 ? epi.rq_scales[0] : epi.rq_scales[p_img];
                                 int8_t *dst = epi.out_i8 + ((size_t)p_img * epi.P + p0) * epi.out_cp + o;
-                                TSB_EPI_DISPATCH(done =, patch_i8_run, v, my_dq, my_bias, epi.leaky, rs, o < epi.out_cp, dst, (uint32_t)epi.out_cp,
-                                                 (uint32_t)(kp.OW * epi.out_cp), rows_live, cols_live);
+                                with_act_flag(act, epi.even, [&](auto a, auto even) {
+                                    done = patch_i8_run<TSB_VAL(a), TSB_VAL(even)>(v, my_dq, my_bias, epi.leaky, rs, o < epi.out_cp, dst, (uint32_t)epi.out_cp,
+                                                                                   (uint32_t)(kp.OW * epi.out_cp), rows_live, cols_live);
+                                });
+                                const int p_top = p0 + (rows_live - 1) * kp.OW + cols_live - 1;
+                                if (epi.tail && done && __any_sync(0xffffffffu, ch_live && ((uint32_t)(p_img * epi.O + o) * (uint32_t)epi.P + (uint32_t)p_top) >= epi.rne_limit))
+                                    fix_tail(epi, taddr0 + (uint32_t)col0, [&](int j) { return ch_live && (j >> 3) < rows_live && (j & 7) < cols_live; },
+                                             [&](int) { return p_img; }, [&](int) { return o; }, [&](int j) { return p0 + (j >> 3) * kp.OW + (j & 7); });
                             }
                         }
                         if (!done) {
@@ -1584,30 +1579,42 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     const bool one_image = npix == 32 && split >= 32;
                     // pixel-major outputs are linear in the pixel index: an image boundary inside the chunk only switches
                     // the requantize scale (at most once when an image has at least 32 pixels)
-                    const bool linear_ok = npix == 32 && kp.P >= 32;
+                    const bool linear_ok = (npix == 32 || EPI != kEpiNhwc) && kp.P >= 32;
                     bool done = false;
-                    if (kp.epi_mode != kEpiGeneric && (kp.epi_mode == kEpiF32Nchw ? one_image : linear_ok)) {
+                    if (EPI != kEpiGeneric && (linear_ok || one_image)) {
                         int v[32];
                         tmem_ld32(taddr0 + (uint32_t)col0, v);
                         tmem_ld_wait();
                         const float rs0 = epi.nscales == 1 ? epi.rq_scales[0] : epi.rq_scales[img0];
                         const float rs1 = epi.nscales == 1 ? rs0 : epi.rq_scales[min(img0 + 1, epi.nscales - 1)];
-                        if (kp.epi_mode == kEpiF32Nchw) {
+                        if constexpr (EPI == kEpiF32Nchw) {
                             if (ch_live) {
                                 float *dst = epi.out_f32 + ((size_t)(img0 * epi.O + o) * (size_t)epi.P + (size_t)p0);
-                                TSB_EPI_DISPATCH(, swap_f32_run, v, my_dq, my_bias, epi.leaky, dst);
+                                if (one_image) with_act(act, [&](auto a) { swap_f32_run<TSB_VAL(a)>(v, my_dq, my_bias, epi.leaky, dst); });
+                                else with_act(act, [&](auto a) { swap_f32_split_run<TSB_VAL(a)>(v, my_dq, my_bias, epi.leaky, dst, npix, split, (uint32_t)((epi.O - 1) * epi.P)); });
                             }
                             done = true;
-                        } else if (kp.epi_mode == kEpiI8Nhwc) {
+                        } else if constexpr (EPI == kEpiI8Nhwc) {
                             int8_t *dst = epi.out_i8 + (size_t)mfirst * epi.out_cp + o;
-                            TSB_EPI_DISPATCH(done =, swap_i8_run, v, my_dq, my_bias, epi.leaky, rs0, rs1, split, o < epi.out_cp, dst, (uint32_t)epi.out_cp);
-                        } else {
+                            with_act_flag(act, epi.even, [&](auto a, auto even) {
+                                done = swap_i8_run<TSB_VAL(a), TSB_VAL(even)>(v, my_dq, my_bias, epi.leaky, rs0, rs1, split, o < epi.out_cp, dst, (uint32_t)epi.out_cp, npix);
+                            });
+                        } else if constexpr (EPI == kEpiNhwc) {
                             const size_t f_off = (size_t)mfirst * epi.O + (ch_live ? o : 0);
                             const float *res = epi.residual ? epi.residual + f_off : nullptr;
                             float *of = epi.out_f32 ? epi.out_f32 + f_off : nullptr;
                             int8_t *oi = epi.out_i8 ? epi.out_i8 + (size_t)mfirst * epi.out_cp + o : nullptr;
-                            TSB_EPI_DISPATCH_SWAPRES(done =, swap_nhwc_run, v, my_dq, my_bias, epi.leaky, res, of, oi, o < epi.out_cp, rs0, rs1, split,
-                                             (uint32_t)epi.O, (uint32_t)epi.out_cp, ch_live);
+                            with_act_flags(act, epi.even, epi.res_after, [&](auto a, auto even, auto after) {
+                                done = swap_nhwc_run<TSB_VAL(a), TSB_VAL(even), TSB_VAL(after)>(v, my_dq, my_bias, epi.leaky, res, of, oi, o < epi.out_cp, rs0, rs1, split,
+                                                                                               (uint32_t)epi.O, (uint32_t)epi.out_cp, ch_live);
+                            });
+                        }
+                        if (EPI != kEpiF32Nchw && epi.tail && done) {       // (one scale: the batch may still have several images)
+                            auto img_of = [&](int j) { return kp.d_P.div(mfirst + j); };
+                            const int last = kp.d_P.div(mfirst + npix - 1), p_last = mfirst + npix - 1 - last * kp.P;
+                            if (__any_sync(0xffffffffu, ch_live && ((uint32_t)(last * epi.O + o) * (uint32_t)epi.P + (uint32_t)p_last) >= epi.rne_limit))
+                                fix_tail(epi, taddr0 + (uint32_t)col0, [&](int j) { return ch_live && j < npix; }, img_of, [&](int) { return o; },
+                                         [&](int j) { return mfirst + j - img_of(j) * kp.P; });
                         }
                     }
                     if (!done) {
@@ -1642,15 +1649,15 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
 }
 
-// Launches one instance (BN, BK, SWAP, MODE, DUAL).
-template <int BN, int BK, bool SWAP, int MODE, bool DUAL>
+// Launches one instance.
+template <int BN, int BK, bool SWAP, int MODE, int EPI, bool DUAL>
 int launch(const Config &cfg, const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mr, const CUtensorMap &mof,
            const CUtensorMap &moi, const KernelParams &kp, const EpiParams &epi, cudaStream_t stream,
            const std::conditional_t<DUAL, DualParams, NoDual> &dual) {
     // The shared-memory limit of a kernel is a per-device attribute: one process may drive several GPUs (one TenniS
     // Workbench per device, each on its own thread), so the "already raised" note is kept per device.
     static std::atomic<uint64_t> configured{0};
-    auto kernel = conv_i8_tc_kernel<BN, BK, SWAP, MODE, DUAL>;
+    auto kernel = conv_i8_tc_kernel<BN, BK, SWAP, MODE, EPI, DUAL>;
     int dev = 0;
     TSB_CUDA(cudaGetDevice(&dev));
     const uint64_t bit = dev >= 0 && dev < 64 ? 1ull << dev : 0;
@@ -1664,15 +1671,30 @@ int launch(const Config &cfg, const CUtensorMap &ma, const CUtensorMap &mb, cons
 }
 
 // The instances of the kernel, in groups that are compiled side by side (one object file of conv_tc_inst.cu per group).
-#define TSB_TC_PART_0(X) X(64, 64, false, kModeGeneral, false) X(128, 64, false, kModeGeneral, false) X(128, 64, true, kModeGeneral, false) X(64, 64, false, kModeRows, false)
-#define TSB_TC_PART_1(X) X(256, 64, false, kModeGeneral, false) X(256, 64, true, kModeGeneral, false) X(64, 128, false, kModeGeneral, false) X(64, 128, false, kModeRows, false)
-#define TSB_TC_PART_2(X) X(128, 128, false, kModeGeneral, false) X(128, 128, true, kModeGeneral, false) X(128, 64, false, kModeRows, false) X(128, 128, false, kModeRows, false)
-#define TSB_TC_PART_3(X) X(256, 128, false, kModeGeneral, false) X(256, 128, true, kModeGeneral, false) X(256, 64, false, kModeRows, false) X(256, 128, false, kModeRows, false)
-#define TSB_TC_PART_4(X) X(64, 64, false, kModePatch, false) X(128, 64, false, kModePatch, false) X(128, 64, true, kModePatch, false) X(256, 64, true, kModePatch, false)
-#define TSB_TC_PART_5(X) X(64, 128, false, kModePatch, false) X(128, 128, false, kModePatch, false) X(128, 128, true, kModePatch, false) X(256, 64, false, kModePatch, false)
-#define TSB_TC_PART_6(X) X(256, 128, false, kModePatch, false) X(256, 128, true, kModePatch, false) X(64, 64, false, kModeGeneral, true) X(64, 128, false, kModeGeneral, true)
-#define TSB_TC_PART_7(X) X(128, 64, false, kModeGeneral, true) X(128, 128, false, kModeGeneral, true) X(256, 64, false, kModeGeneral, true) X(256, 128, false, kModeGeneral, true)
-#define TSB_TC_ALL(X) TSB_TC_PART_0(X) TSB_TC_PART_1(X) TSB_TC_PART_2(X) TSB_TC_PART_3(X) TSB_TC_PART_4(X) TSB_TC_PART_5(X) TSB_TC_PART_6(X) TSB_TC_PART_7(X)
+// X(BN, BK, SWAP, MODE, EPI, DUAL)
+#define TSB_TC_NORMAL(X, BN_, BK_, MODE_)                                                                                    \
+    X(BN_, BK_, false, MODE_, kEpiGeneric, false) X(BN_, BK_, false, MODE_, kEpiF32Nchw, false)                             \
+    X(BN_, BK_, false, MODE_, kEpiI8Nhwc, false) X(BN_, BK_, false, MODE_, kEpiStaged, false)
+#define TSB_TC_SWAPPED(X, BN_, BK_)                                                                                          \
+    X(BN_, BK_, true, kModeGeneral, kEpiGeneric, false) X(BN_, BK_, true, kModeGeneral, kEpiF32Nchw, false)                 \
+    X(BN_, BK_, true, kModeGeneral, kEpiI8Nhwc, false) X(BN_, BK_, true, kModeGeneral, kEpiNhwc, false)                     \
+    X(BN_, BK_, true, kModePatch, kEpiGeneric, false) X(BN_, BK_, true, kModePatch, kEpiF32Nchw, false)                     \
+    X(BN_, BK_, true, kModePatch, kEpiI8Nhwc, false)
+#define TSB_TC_PAIR(X, BN_, BK_) X(BN_, BK_, false, kModeGeneral, kEpiStaged, true) X(BN_, BK_, false, kModeGeneral, kEpiI8Nhwc, true)
+#define TSB_TC_PART_0(X) TSB_TC_NORMAL(X, 64, 64, kModeGeneral) TSB_TC_NORMAL(X, 64, 128, kModeGeneral) TSB_TC_NORMAL(X, 64, 64, kModePatch)
+#define TSB_TC_PART_1(X) TSB_TC_NORMAL(X, 128, 64, kModeGeneral) TSB_TC_NORMAL(X, 128, 128, kModeGeneral) TSB_TC_NORMAL(X, 64, 128, kModePatch)
+#define TSB_TC_PART_2(X) TSB_TC_NORMAL(X, 256, 64, kModeGeneral) TSB_TC_NORMAL(X, 256, 128, kModeGeneral)
+#define TSB_TC_PART_3(X) TSB_TC_NORMAL(X, 128, 64, kModePatch) TSB_TC_NORMAL(X, 128, 128, kModePatch)
+#define TSB_TC_PART_4(X) TSB_TC_NORMAL(X, 256, 64, kModePatch) TSB_TC_NORMAL(X, 256, 128, kModePatch)
+#define TSB_TC_PART_5(X) TSB_TC_NORMAL(X, 64, 64, kModeRows) TSB_TC_NORMAL(X, 128, 64, kModeRows) TSB_TC_NORMAL(X, 256, 64, kModeRows)
+#define TSB_TC_PART_6(X) TSB_TC_NORMAL(X, 64, 128, kModeRows) TSB_TC_NORMAL(X, 128, 128, kModeRows) TSB_TC_NORMAL(X, 256, 128, kModeRows)
+#define TSB_TC_PART_7(X) TSB_TC_SWAPPED(X, 128, 64) TSB_TC_SWAPPED(X, 128, 128)
+#define TSB_TC_PART_8(X) TSB_TC_SWAPPED(X, 256, 64) TSB_TC_SWAPPED(X, 256, 128)
+#define TSB_TC_PART_9(X)                                                                                                     \
+    TSB_TC_PAIR(X, 64, 64) TSB_TC_PAIR(X, 64, 128) TSB_TC_PAIR(X, 128, 64) TSB_TC_PAIR(X, 128, 128) TSB_TC_PAIR(X, 256, 64) TSB_TC_PAIR(X, 256, 128)
+#define TSB_TC_ALL(X)                                                                                                        \
+    TSB_TC_PART_0(X) TSB_TC_PART_1(X) TSB_TC_PART_2(X) TSB_TC_PART_3(X) TSB_TC_PART_4(X) TSB_TC_PART_5(X) TSB_TC_PART_6(X)  \
+    TSB_TC_PART_7(X) TSB_TC_PART_8(X) TSB_TC_PART_9(X)
 
 }  // namespace tc
 }  // namespace tsb
