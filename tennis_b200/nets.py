@@ -85,6 +85,7 @@ class QuantResNet:
         # the projection shortcut of a stage's first block runs inside the launch of the block's last convolution
         # (tsb_conv2d_i8_run_projected); False: as a launch of its own whose fp32 output is that convolution's residual
         self.fuse_projection = fuse_projection
+        self.fuse_concat = False
         self.lib = _lib.load()
         dev = self.dev
         self.convs = []
@@ -100,6 +101,41 @@ class QuantResNet:
         self.buffers = {}
         self.calibrated = False
         self.launch_log = None
+        # forward(): the pass as bound library calls, laid out by the first pass after a calibration (every tensor between
+        # input and output is the network's own, so only the input's address changes)
+        self.steps = None
+        self.recording = None
+
+    def _step(self, call):
+        """Runs a bound library call, and notes it when a pass is being laid out."""
+        call(ops._stream_ptr())
+        if self.recording is not None:
+            self.recording.append(call)
+
+    def _call(self, fn, args, keep):
+        self._step(ops.Call(fn, args, keep))
+
+    def _replay(self, x, lay_out):
+        """One pass: the staging quantize of x, then the bound calls; lay_out(x) is the pass as plain code, which the first
+        call records.  (A ResNet-50 pass of one image is 60 launches: 0.64 ms as plain code, which the host bounds, and 0.40 ms
+        bound, which the GPU bounds.)"""
+        fused = (self.fuse_projection, self.fuse_concat)
+        if self.steps is None or self.steps[2] != fused or self.launch_log is not None:
+            self.recording = []
+            try:
+                out = lay_out(x)
+                self.steps = (self.recording, out, fused)
+            finally:
+                self.recording = None
+            return out
+        calls, out, _ = self.steps
+        self.convs[0]["plan"].quantize_input(x, self.input_scale_arr)
+        stream = ops._stream_ptr()
+        for call in calls:
+            status = call.fn(*call.args, stream)
+            if status:
+                check(status)
+        return out
 
     # ---- buffers ------------------------------------------------------------------------------------------------
     def _i8(self, key, pixels_hw, channels):
@@ -122,18 +158,17 @@ class QuantResNet:
         out_i8 = self._i8(key + ".i8", c["oh"], c["o"]) if want_i8 else None
         out_f32 = self._f32(key + ".f32", c["oh"], c["o"]) if want_f32 else None
 
-        def launch():
-            L["plan"].run(None if staged else x_i8, LAYOUT_STAGED if staged else LAYOUT_NHWC_PAD, L["dq"], bias=L["bias"],
-                          residual=residual, activation=act, leaky=leaky, out_f32=out_f32, out_f32_layout=LAYOUT_NHWC_PAD,
-                          out_i8=out_i8, out_i8_layout=LAYOUT_NHWC_PAD,
-                          requant_scales=L["out_scale_arr"] if want_i8 else None, residual_after_activation=residual_after)
-        launch()
+        call = L["plan"].bind_run(None if staged else x_i8, LAYOUT_STAGED if staged else LAYOUT_NHWC_PAD, L["dq"], bias=L["bias"],
+                                  residual=residual, activation=act, leaky=leaky, out_f32=out_f32, out_f32_layout=LAYOUT_NHWC_PAD,
+                                  out_i8=out_i8, out_i8_layout=LAYOUT_NHWC_PAD,
+                                  requant_scales=L["out_scale_arr"] if want_i8 else None, residual_after_activation=residual_after)
+        self._step(call)
         if self.launch_log is not None:      # layer_times(): every convolution launch of a pass, replayable
             out_bytes = (out_i8.numel() if want_i8 else 0) + (4 * self.batch * c["oh"] * c["oh"] * c["o"] if want_f32 else 0)
             in_bytes = self.batch * c["h"] * c["h"] * ops.padded_channels(c["c"]) + c["o"] * c["c"] * c["k"] * c["k"] + 8 * c["o"]
             if residual is not None:
                 in_bytes += 4 * self.batch * c["oh"] * c["oh"] * c["o"]
-            self.launch_log.append(dict(name=c["name"], launch=launch, ops=2 * self.batch * c["o"] * c["oh"] * c["oh"] * c["c"] * c["k"] * c["k"],
+            self.launch_log.append(dict(name=c["name"], launch=lambda: call(ops._stream_ptr()), ops=2 * self.batch * c["o"] * c["oh"] * c["oh"] * c["c"] * c["k"] * c["k"],
                                         bytes=in_bytes + out_bytes, k=c["k"], c=c["c"], o=c["o"], size=c["oh"], stride=c["stride"],
                                         residual=residual is not None, fp32_out=bool(want_f32), int8_out=bool(want_i8)))
         return out_i8, out_f32
@@ -145,15 +180,14 @@ class QuantResNet:
         out_i8 = self._i8(key + ".i8", c["oh"], c["o"])
         out_f32 = self._f32(key + ".f32", c["oh"], c["o"])
 
-        def launch():
-            L["plan"].run_projected(x_i8, S["plan"], x_proj, L["dq"], S["dq"], bias=L["bias"], shortcut_bias=S["bias"],
-                                    activation=act, out_f32=out_f32, out_i8=out_i8, requant_scales=L["out_scale_arr"])
-        launch()
+        call = L["plan"].bind_projected(x_i8, S["plan"], x_proj, L["dq"], S["dq"], bias=L["bias"], shortcut_bias=S["bias"],
+                                        activation=act, out_f32=out_f32, out_i8=out_i8, requant_scales=L["out_scale_arr"])
+        self._step(call)
         if self.launch_log is not None:
             px = self.batch * c["oh"] * c["oh"]
             in_bytes = (self.batch * c["h"] * c["h"] * ops.padded_channels(c["c"]) + c["o"] * c["c"] * c["k"] * c["k"] + 8 * c["o"] +
                         self.batch * cs["h"] * cs["h"] * ops.padded_channels(cs["c"]) // (cs["stride"] ** 2) + c["o"] * cs["c"] + 8 * c["o"])
-            self.launch_log.append(dict(name=c["name"] + "+proj", launch=launch, ops=2 * px * c["o"] * (c["c"] * c["k"] * c["k"] + cs["c"]),
+            self.launch_log.append(dict(name=c["name"] + "+proj", launch=lambda: call(ops._stream_ptr()), ops=2 * px * c["o"] * (c["c"] * c["k"] * c["k"] + cs["c"]),
                                         bytes=in_bytes + out_i8.numel() + 4 * px * c["o"], k=c["k"], c=c["c"] + cs["c"], o=c["o"],
                                         size=c["oh"], stride=c["stride"], residual=False, fp32_out=True, int8_out=True))
         return out_i8, out_f32
@@ -190,6 +224,7 @@ class QuantResNet:
     def calibrate(self, x):
         """x: fp32 NCHW sample batch on the device.  Fixes every activation scale; returns them as a dict."""
         spec = self.spec
+        self.steps = None
         amax = float(x.abs().max())
         self.input_scale = np.float32(127.0) / np.float32(amax if amax > 0 else 1.0)
         self._set_in_scale(0, self.input_scale)
@@ -236,13 +271,16 @@ class QuantResNet:
         s_i8, _ = self._conv(0, None, "stem", ACT_RELU, staged=True)
         c = L["spec"]
         pooled = self._i8("stem.pool", spec["stem_pooled"], c["o"])
-        check(self.lib.tsb_maxpool_i8_nhwc(s_i8.data_ptr(), pooled.data_ptr(), self.batch, c["oh"], c["oh"], c["o"], 3, 2, 1, 0, 1, 0,
-                                           ops._stream_ptr()))
+        self._call(self.lib.tsb_maxpool_i8_nhwc, (s_i8.data_ptr(), pooled.data_ptr(), self.batch, c["oh"], c["oh"], c["o"], 3, 2, 1, 0, 1, 0),
+                   (s_i8, pooled))
         return pooled
 
     def forward(self, x):
         """x: fp32 NCHW [batch, 3, image, image] on the device -> fp32 logits [batch, classes]."""
         assert self.calibrated, "call calibrate() first"
+        return self._replay(x, self._pass)
+
+    def _pass(self, x):
         spec = self.spec
         x_i8 = self._forward_stem(x)
         x_f32 = None
@@ -258,12 +296,14 @@ class QuantResNet:
                 else:
                     sc = x_f32
                 x_i8, x_f32 = self._conv(b["conv3"], bb, b["name"] + ".y", ACT_RELU, want_i8=True, want_f32=True, residual=sc)
-        feat = self.buffers.setdefault("feat", torch.empty((self.batch, spec["features"]), dtype=torch.float32, device=self.dev))
-        logits = self.buffers.setdefault("logits", torch.empty((self.batch, spec["classes"]), dtype=torch.float32, device=self.dev))
+        for key, width in (("feat", spec["features"]), ("logits", spec["classes"])):
+            if key not in self.buffers:
+                self.buffers[key] = torch.empty((self.batch, width), dtype=torch.float32, device=self.dev)
+        feat, logits = self.buffers["feat"], self.buffers["logits"]
         P = spec["final_size"] * spec["final_size"]
-        check(self.lib.tsb_global_avgpool_f32_nhwc(x_f32.data_ptr(), feat.data_ptr(), self.batch, P, spec["features"], ops._stream_ptr()))
-        check(self.lib.tsb_inner_prod_f32(feat.data_ptr(), self.fc_w.data_ptr(), self.fc_b.data_ptr(), logits.data_ptr(), self.batch,
-                                          spec["features"], spec["classes"], ops._stream_ptr()))
+        self._call(self.lib.tsb_global_avgpool_f32_nhwc, (x_f32.data_ptr(), feat.data_ptr(), self.batch, P, spec["features"]), (x_f32, feat))
+        self._call(self.lib.tsb_inner_prod_f32, (feat.data_ptr(), self.fc_w.data_ptr(), self.fc_b.data_ptr(), logits.data_ptr(), self.batch,
+                                                 spec["features"], spec["classes"]), (feat, self.fc_w, self.fc_b, logits))
         return logits
 
     def status(self):
@@ -388,21 +428,19 @@ class QuantCSPDarknet(QuantResNet):
         p_first, p_rest = self.halves[idx]
         out_i8 = self._i8(key + ".i8", c["oh"], c["o"])
 
-        def launch():
-            p_rest.run_concat(rest, p_first, first, L["dq"], bias=L["bias"], activation=act, leaky=leaky, out_i8=out_i8,
-                              requant_scales=L["out_scale_arr"])
-        launch()
+        call = p_rest.bind_concat(rest, p_first, first, L["dq"], bias=L["bias"], activation=act, leaky=leaky, out_i8=out_i8,
+                                  requant_scales=L["out_scale_arr"])
+        self._step(call)
         if self.launch_log is not None:
             px = self.batch * c["oh"] * c["oh"]
-            self.launch_log.append(dict(name=c["name"] + "+concat", launch=launch, ops=2 * px * c["o"] * c["c"],
+            self.launch_log.append(dict(name=c["name"] + "+concat", launch=lambda: call(ops._stream_ptr()), ops=2 * px * c["o"] * c["c"],
                                         bytes=px * ops.padded_channels(c["c"]) + c["o"] * c["c"] + 8 * c["o"] + out_i8.numel(),
                                         k=1, c=c["c"], o=c["o"], size=c["oh"], stride=1, residual=False, fp32_out=False, int8_out=True))
         return out_i8
 
     def _concat(self, a, ca, b, cb, key, size):
         out = self._i8(key, size, ca + cb)
-        check(self.lib.tsb_concat_i8_nhwc(a.data_ptr(), ca, b.data_ptr(), cb, out.data_ptr(), self.batch * size * size,
-                                          ops._stream_ptr()))
+        self._call(self.lib.tsb_concat_i8_nhwc, (a.data_ptr(), ca, b.data_ptr(), cb, out.data_ptr(), self.batch * size * size), (a, b, out))
         return out
 
     def _scale(self, m):
@@ -464,6 +502,7 @@ class QuantCSPDarknet(QuantResNet):
         return cur
 
     def calibrate(self, x):
+        self.steps = None
         out = self._walk(x, calibrate=True)
         self.calibrated = True
         torch.cuda.synchronize()
@@ -473,7 +512,7 @@ class QuantCSPDarknet(QuantResNet):
     def forward(self, x):
         """x: fp32 NCHW [batch, 3, image, image] on the device -> int8 NHWC_PAD feature map of the last stage."""
         assert self.calibrated, "call calibrate() first"
-        return self._walk(x, calibrate=False)
+        return self._replay(x, lambda x: self._walk(x, calibrate=False))
 
 
 def _main():

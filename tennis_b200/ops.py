@@ -26,13 +26,20 @@ class EjectionException(RuntimeError):
     """What TS_LOG_ERROR << ... << eject raises in the reference (include/utils/log.h:162-166)."""
 
 
+# The raw handle of the current stream.  A small convolution takes the GPU 4 us and the driver 3 us to launch;
+# torch.cuda.current_stream() builds a Stream object for 3 us more, these two calls take 0.2 us.
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
+_current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is None:
+        return _current_raw_stream(_current_device())
+    return stream.cuda_stream
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def padded_channels(c):
@@ -102,6 +109,7 @@ class Quantize(Operator):
     def init(self):
         super().init()
         self.scales = [float(v) for v in np.asarray(self.get("quantize_scale"), dtype=np.float32).reshape(-1)]
+        self._scale_array = float_array(self.scales)
 
     def infer(self, inputs):
         _auto_check(len(inputs) == 1, "stack.size() == 1")
@@ -118,8 +126,55 @@ class Quantize(Operator):
         y = torch.empty(x.shape, dtype=torch.int8, device=x.device)
         lib = _lib.load()
         fn = lib.tsb_quantize_f32_i8 if x.dtype == torch.float32 else lib.tsb_quantize_f64_i8
-        check(fn(_ptr(x), _ptr(y), x.numel(), float_array(self.scales), len(self.scales), _stream_ptr(stream)))
+        status = fn(x.data_ptr(), y.data_ptr(), x.numel(), self._scale_array, len(self._scale_array), _stream_ptr(stream))
+        if status:
+            check(status)
         return y
+
+
+class Call:
+    """A library call with every argument but the stream bound, and what those arguments point to kept alive."""
+
+    __slots__ = ("fn", "args", "keep")
+
+    def __init__(self, fn, args, keep):
+        self.fn, self.args, self.keep = fn, args, keep
+
+    def __call__(self, stream_ptr):
+        status = self.fn(*self.args, stream_ptr)
+        if status:
+            check(status)
+
+
+def _scales_of(values):
+    return values if isinstance(values, ctypes.Array) else float_array(values)
+
+
+def _epilogue(dq, bias, residual, activation, leaky, out_f32, out_f32_layout, out_i8, out_i8_layout, requant_scales, out_acc,
+              residual_after_activation):
+    """The ConvEpilogue of these tensors (it refers to requant_scales, a ctypes array, which the caller keeps)."""
+    e = ConvEpilogue()
+    e.dequantize_scales = dq.data_ptr()
+    e.activation = int(activation)
+    e.leaky_scale = leaky
+    if residual_after_activation:
+        e.residual_after_activation = 1
+    if bias is not None:
+        e.bias = bias.data_ptr()
+    if residual is not None:
+        e.residual = residual.data_ptr()
+    if out_f32 is not None:
+        e.out_f32 = out_f32.data_ptr()
+    e.out_f32_layout = out_f32_layout
+    if out_i8 is not None:
+        e.out_i8 = out_i8.data_ptr()
+    e.out_i8_layout = out_i8_layout
+    if requant_scales is not None:
+        e.requant_scales_host = requant_scales
+        e.n_requant_scales = len(requant_scales)
+    if out_acc is not None:
+        e.out_acc = out_acc.data_ptr()
+    return e
 
 
 class ConvPlan:
@@ -127,7 +182,7 @@ class ConvPlan:
 
     def __init__(self, xshape, wshape, pad, stride, dilation, padding_value=0.0, kernel=KERNEL_AUTO, device="cuda",
                  mma_orientation=0, raw_row_mode=0, patch_mode=0):
-        lib = _lib.load()
+        lib = self._lib = _lib.load()
         d = ConvDesc()
         d.mma_orientation, d.raw_row_mode, d.patch_mode = int(mma_orientation), int(raw_row_mode), int(patch_mode)
         d.n, d.c, d.h, d.w = [int(v) for v in xshape]
@@ -167,80 +222,68 @@ class ConvPlan:
     def quantize_input(self, x_f32, scales, stream=None):
         """fp32 NCHW -> the plan's staged int8 input; run() is then called with x=None, x_layout=LAYOUT_STAGED."""
         arr = scales if not isinstance(scales, (list, tuple)) else float_array(scales)
-        check(_lib.load().tsb_conv2d_i8_quantize_input(self.handle, _ptr(x_f32), arr, len(arr), _ptr(self.workspace),
-                                                       self.ws_bytes, _stream_ptr(stream)))
+        status = self._lib.tsb_conv2d_i8_quantize_input(self.handle, x_f32.data_ptr(), arr, len(arr), self.workspace.data_ptr(),
+                                                        self.ws_bytes, _stream_ptr(stream))
+        if status:
+            check(status)
 
     def run(self, x, x_layout, dq, bias=None, residual=None, activation=ACT_NONE, leaky=0.0, out_f32=None,
             out_f32_layout=LAYOUT_NCHW, out_i8=None, out_i8_layout=LAYOUT_NCHW, requant_scales=None, out_acc=None,
             stream=None, residual_after_activation=False):
-        e = ConvEpilogue()
-        e.residual_after_activation = 1 if residual_after_activation else 0
-        e.dequantize_scales = dq.data_ptr()
-        e.bias = bias.data_ptr() if bias is not None else None
-        e.residual = residual.data_ptr() if residual is not None else None
-        e.activation = int(activation)
-        e.leaky_scale = float(leaky)
-        e.out_f32 = out_f32.data_ptr() if out_f32 is not None else None
-        e.out_f32_layout = int(out_f32_layout)
-        e.out_i8 = out_i8.data_ptr() if out_i8 is not None else None
-        e.out_i8_layout = int(out_i8_layout)
-        keep = None
-        if requant_scales is not None:
-            keep = requant_scales if isinstance(requant_scales, ctypes.Array) else float_array(requant_scales)
-            e.requant_scales_host = keep
-            e.n_requant_scales = len(requant_scales)
-        e.out_acc = out_acc.data_ptr() if out_acc is not None else None
-        check(_lib.load().tsb_conv2d_i8_run(self.handle, _ptr(x), int(x_layout), ctypes.byref(e), _ptr(self.workspace),
-                                            self.ws_bytes, _stream_ptr(stream)))
+        rq = None if requant_scales is None else _scales_of(requant_scales)
+        e = _epilogue(dq, bias, residual, activation, leaky, out_f32, out_f32_layout, out_i8, out_i8_layout, rq, out_acc,
+                      residual_after_activation)
+        status = self._lib.tsb_conv2d_i8_run(self.handle, None if x is None else x.data_ptr(), x_layout, e, self.workspace.data_ptr(),
+                                             self.ws_bytes, _stream_ptr(stream))
+        if status:
+            check(status)
+
+    def bind_run(self, x, x_layout, dq, bias=None, residual=None, activation=ACT_NONE, leaky=0.0, out_f32=None,
+                 out_f32_layout=LAYOUT_NCHW, out_i8=None, out_i8_layout=LAYOUT_NCHW, requant_scales=None,
+                 residual_after_activation=False):
+        """run() with these tensors as a Call, for programs that launch the same layer on the same buffers again and again."""
+        rq = None if requant_scales is None else _scales_of(requant_scales)
+        e = _epilogue(dq, bias, residual, activation, leaky, out_f32, out_f32_layout, out_i8, out_i8_layout, rq, None,
+                      residual_after_activation)
+        args = (self.handle, _ptr(x), int(x_layout), ctypes.byref(e), self.workspace.data_ptr(), self.ws_bytes)
+        return Call(self._lib.tsb_conv2d_i8_run, args, (self, e, rq, x, dq, bias, residual, out_f32, out_i8))
+
+    def bind_projected(self, x, shortcut, x_shortcut, dq, shortcut_dq, bias=None, shortcut_bias=None, activation=ACT_NONE,
+                       leaky=0.0, out_f32=None, out_i8=None, requant_scales=None, residual_after_activation=False,
+                       tile_channels=0):
+        """run_projected() with these tensors as a Call."""
+        rq = None if requant_scales is None else _scales_of(requant_scales)
+        e = _epilogue(dq, bias, None, activation, leaky, out_f32, LAYOUT_NHWC_PAD, out_i8, LAYOUT_NHWC_PAD, rq, None,
+                      residual_after_activation)
+        args = (self.handle, _ptr(x), shortcut.handle, _ptr(x_shortcut), _ptr(shortcut_dq), _ptr(shortcut_bias), ctypes.byref(e),
+                int(tile_channels), self.workspace.data_ptr(), self.ws_bytes)
+        return Call(self._lib.tsb_conv2d_i8_run_projected, args,
+                    (self, shortcut, e, rq, x, x_shortcut, dq, shortcut_dq, bias, shortcut_bias, out_f32, out_i8))
 
     def run_projected(self, x, shortcut, x_shortcut, dq, shortcut_dq, bias=None, shortcut_bias=None, activation=ACT_NONE,
                       leaky=0.0, out_f32=None, out_i8=None, requant_scales=None, stream=None,
                       residual_after_activation=False, tile_channels=0):
         """This convolution with the 1x1 projection `shortcut` (another ConvPlan, its weights set) as its residual, in
         one launch (tsb_conv2d_i8_run_projected): NHWC_PAD int8 inputs, pixel-major fp32 / NHWC_PAD int8 outputs."""
-        e = ConvEpilogue()
-        e.residual_after_activation = 1 if residual_after_activation else 0
-        e.dequantize_scales = dq.data_ptr()
-        e.bias = bias.data_ptr() if bias is not None else None
-        e.residual = None
-        e.activation = int(activation)
-        e.leaky_scale = float(leaky)
-        e.out_f32 = out_f32.data_ptr() if out_f32 is not None else None
-        e.out_f32_layout = LAYOUT_NHWC_PAD
-        e.out_i8 = out_i8.data_ptr() if out_i8 is not None else None
-        e.out_i8_layout = LAYOUT_NHWC_PAD
-        keep = None
-        if requant_scales is not None:
-            keep = requant_scales if isinstance(requant_scales, ctypes.Array) else float_array(requant_scales)
-            e.requant_scales_host = keep
-            e.n_requant_scales = len(requant_scales)
-        check(_lib.load().tsb_conv2d_i8_run_projected(
-            self.handle, _ptr(x), shortcut.handle, _ptr(x_shortcut), _ptr(shortcut_dq),
-            _ptr(shortcut_bias) if shortcut_bias is not None else None, ctypes.byref(e), int(tile_channels),
-            _ptr(self.workspace), self.ws_bytes, _stream_ptr(stream)))
+        self.bind_projected(x, shortcut, x_shortcut, dq, shortcut_dq, bias, shortcut_bias, activation, leaky, out_f32, out_i8,
+                            requant_scales, residual_after_activation, tile_channels)(_stream_ptr(stream))
+
+    def bind_concat(self, x, first, x_first, dq, bias=None, activation=ACT_NONE, leaky=0.0, out_f32=None, out_i8=None,
+                    requant_scales=None, tile_channels=0):
+        """run_concat() with these tensors as a Call."""
+        rq = None if requant_scales is None else _scales_of(requant_scales)
+        e = _epilogue(dq, bias, None, activation, leaky, out_f32, LAYOUT_NHWC_PAD, out_i8, LAYOUT_NHWC_PAD, rq, None, False)
+        args = (self.handle, _ptr(x), first.handle, _ptr(x_first), ctypes.byref(e), int(tile_channels), self.workspace.data_ptr(),
+                self.ws_bytes)
+        return Call(self._lib.tsb_conv2d_i8_run_concat, args, (self, first, e, rq, x, x_first, dq, bias, out_f32, out_i8))
 
     def run_concat(self, x, first, x_first, dq, bias=None, activation=ACT_NONE, leaky=0.0, out_f32=None, out_i8=None,
                    requant_scales=None, stream=None, tile_channels=0):
         """The convolution over concat(x_first, x) along channels in one launch (tsb_conv2d_i8_run_concat): `first` holds the
         weight columns of the leading channels (a 1x1 plan), this plan the rest; NHWC_PAD int8 inputs quantized with the
         same scales, pixel-major fp32 / NHWC_PAD int8 outputs."""
-        e = ConvEpilogue()
-        e.dequantize_scales = dq.data_ptr()
-        e.bias = bias.data_ptr() if bias is not None else None
-        e.residual = None
-        e.activation = int(activation)
-        e.leaky_scale = float(leaky)
-        e.out_f32 = out_f32.data_ptr() if out_f32 is not None else None
-        e.out_f32_layout = LAYOUT_NHWC_PAD
-        e.out_i8 = out_i8.data_ptr() if out_i8 is not None else None
-        e.out_i8_layout = LAYOUT_NHWC_PAD
-        keep = None
-        if requant_scales is not None:
-            keep = requant_scales if isinstance(requant_scales, ctypes.Array) else float_array(requant_scales)
-            e.requant_scales_host = keep
-            e.n_requant_scales = len(requant_scales)
-        check(_lib.load().tsb_conv2d_i8_run_concat(self.handle, _ptr(x), first.handle, _ptr(x_first), ctypes.byref(e),
-                                                   int(tile_channels), _ptr(self.workspace), self.ws_bytes, _stream_ptr(stream)))
+        self.bind_concat(x, first, x_first, dq, bias, activation, leaky, out_f32, out_i8, requant_scales,
+                         tile_channels)(_stream_ptr(stream))
 
     def status(self, stream=None):
         check(_lib.load().tsb_conv2d_i8_status(self.handle, _ptr(self.workspace), _stream_ptr(stream)))
@@ -336,24 +379,27 @@ class Conv2DQuantized(Operator):
         return [("float32", (x.shape[0], OH, OW, w.shape[0]))]
 
     def run(self, inputs, stream=None, out_acc=None):
-        proto = self.infer(inputs)[0]
-        if self.format != "NCHW":
-            raise EjectionException("Conv2D_quantized only support NCHW")  # conv2d_quantized_core.cpp:131-133
-        x, w = inputs
-        x = x.contiguous()
-        pad, stride, dil = self._geometry()
-        key = (tuple(x.shape), tuple(w.shape), w.data_ptr())
-        plan = self._plans.get(key)
+        plan = None
+        if len(inputs) == 2:
+            x, w = inputs
+            # a plan was made for these shapes and types only after they had passed every check
+            key = (x.shape, w.shape, w.data_ptr(), x.dtype, w.dtype, x.device)
+            plan = self._plans.get(key)
         if plan is None:
+            self.infer(inputs)
+            if self.format != "NCHW":
+                raise EjectionException("Conv2D_quantized only support NCHW")  # conv2d_quantized_core.cpp:131-133
+            pad, strides, dil = self._geometry()
             try:
-                plan = ConvPlan(x.shape, w.shape, pad, stride, dil, self.padding_value, self._kernel, x.device)
+                plan = ConvPlan(x.shape, w.shape, pad, strides, dil, self.padding_value, self._kernel, x.device)
             except TsbError as e:
                 raise EjectionException(e.message)
             plan.set_weights(w, stream)
             self._plans[key] = plan
         if self._dq_dev is None or self._dq_dev.device != x.device:
             self._dq_dev = torch.from_numpy(self.dequantize_scales).to(x.device)
-        out = torch.empty(proto[1], dtype=torch.float32, device=x.device)
+        x = x.contiguous()
+        out = torch.empty(plan.out_shape, dtype=torch.float32, device=x.device)
         plan.run(x, LAYOUT_NCHW, self._dq_dev, out_f32=out, out_acc=out_acc, stream=stream)
         return out
 
