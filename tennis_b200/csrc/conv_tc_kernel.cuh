@@ -854,6 +854,27 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             tap16[t] = (uint32_t)((kh * kp.dh * kp.patch_pw + kw * kp.dw) * BK) >> 4;
         }
     }
+    // How many warps issue MMAs, each for every such tile of the CTA.  One where tiles share state that one thread has to order -- a
+    // raw-row stage shared by the segments of an output row, or resident weights that are replaced inside this CTA's tile
+    // range -- and where the ring of stages has no room for a tile of each issuer.
+    // Each issuer has a ring of stages of its own (stages [i * kStages / issuers, ...) for issuer i), which the producer fills for
+    // that issuer's tiles.  A barrier wait names a phase by its parity only; in a ring that nobody else consumes, an issuer
+    // has itself seen the round before the one it waits for.  (With one ring for both, an issuer could arrive at a stage while the
+    // other issuer's tile of the round before was still being loaded -- loads complete out of order -- and pass its wait.)
+    int issuers = 1;
+    if (my_tiles > 1 && warp <= kIssuers) {
+        const int spt = MODE == kModePatch ? kp.Cp / BK : (MODE == kModeRows ? 1 : (k_iters + k_sc) / kp.kgroup);   // stages a tile consumes
+        bool shared_state = MODE == kModeRows && kp.rows_segs > 1;
+        if (kp.b_resident && kp.num_n_tiles > 1) {
+            int first_m, first_n, last_m, last_n;
+            decode(0, first_m, first_n);
+            decode(my_tiles - 1, last_m, last_n);
+            shared_state = shared_state || first_n != last_n;
+        }
+        // (an issuer must also own its accumulator buffers: with a single logical buffer one thread takes every tile)
+        if (!shared_state && kStages >= kIssuers * spt && !(DUAL && nbuf < kIssuers)) issuers = kIssuers;
+    }
+    const int ring = issuers > 1 ? kStages / kIssuers : kStages;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -863,10 +884,17 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
-            int stage = 0; uint32_t phase = 0;
+            int stage = 0, stage_lo = 0, stage_alt = ring;                  // absolute stage, first stage of its ring; the other ring's
+            uint32_t phase = 0, phase_alt = 0;
+            auto next_stage = [&]() { if (++stage == stage_lo + ring) { stage = stage_lo; phase ^= 1u; } };
             bool ok = true;
             int cur_n = -1, w_loads = 0;
             for (int i = 0; i < my_tiles && ok; ++i) {
+                if (i > 0 && issuers > 1) {                                 // the next tile is the other issuer's
+                    const int s = stage; stage = stage_alt; stage_alt = s;
+                    const uint32_t p = phase; phase = phase_alt; phase_alt = p;
+                    stage_lo = ring - stage_lo;
+                }
                 TSB_TRACE(i, 0);
                 int m_tile, n_tile;
                 decode(i, m_tile, n_tile);
@@ -901,7 +929,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         }
                         mbar_arrive_expect_tx(bar_full + 8 * stage, kp.patch_bytes);
                         tma_load_4d(base + stage * kp.stage_bytes, &map_a, bar_full + 8 * stage, cb, w0, h0, p_img);
-                        if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                        next_stage();
                     }
                 } else if (MODE == kModeRows) {
                     // One copy per output row (per run of its segments that this CTA owns): the staged bytes from the
@@ -923,7 +951,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         bulk_load(base + stage * kp.stage_bytes,
                                   kp.rows_x + r_img * kp.rows_stride_n + ih_lo * kp.rows_stride_h + (long long)seg * (PIX * 16),
                                   bytes, bar_full + 8 * stage);
-                        if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                        next_stage();
                     }
                 } else {
                     int gk = 0;   // K block inside the current stage
@@ -944,7 +972,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                             if (!kp.b_resident) tma_load_2d(sw, &dual.map_b2, bar_full + 8 * stage, cb, n_tile * CH);
                             if (++gk == kp.kgroup) {
                                 gk = 0;
-                                if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                                next_stage();
                             }
                         }
                     }
@@ -969,7 +997,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                                     tma_load_2d(sw, &map_b, bar_full + 8 * stage, (kh * kp.KW + kw) * kp.Cp + cb, n_tile * CH);
                                 if (++gk == kp.kgroup) {
                                     gk = 0;
-                                    if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                                    next_stage();
                                 }
                             }
                 }
@@ -989,9 +1017,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         // MMAs is not hidden behind the tensor core's work on the earlier one (measured: ~125 cycles per MMA at N = 64,
         // ~190 at N = 256).  So kIssuers warps issue, each for every kIssuers-th tile of the CTA: while one computes
         // descriptors, waits and commits, the tensor core runs the other's MMAs.  A tile's stages, accumulator buffer and
-        // barriers belong to the issuer of that tile alone.  Where tiles share state that one thread has to order -- a
-        // raw-row stage shared by the segments of an output row, or resident weights that are replaced inside this CTA's
-        // tile range -- the first issuer takes every tile.
+        // barriers belong to the issuer of that tile alone.
         if (lane == 0) {
             constexpr uint32_t idesc = instr_desc<BN>();
             constexpr uint64_t dhi = smem_desc_hi<BK>(8 * BK);
@@ -1001,24 +1027,8 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const int resident = kp.b_resident;
             bool ok = true;
             int rows_seg_first = 0;
-            int first_m = 0, first_n = 0, last_m = 0, last_n = 0;
-            if (my_tiles > 0) { decode(0, first_m, first_n); decode(my_tiles - 1, last_m, last_n); }
-            // pipeline stages a tile consumes
-            const int spt = MODE == kModePatch ? kp.Cp / BK : (MODE == kModeRows ? 1 : (k_iters + k_sc) / kp.kgroup);
-            // A barrier wait names a phase by its parity only, so a waiter must never be two rounds of the stage ring away
-            // from the phase it means.  With several issuers that holds when the ring has room for one tile of each
-            // (kStages >= issuers * spt): the round before the one an issuer waits for then lies in tiles that were
-            // loaded before its own previous tile, whose loads it has seen complete.
-            const bool shared_state = (MODE == kModeRows && kp.rows_segs > 1) || (resident && first_n != last_n);
-            // (an issuer must also own its accumulator buffers: with a single logical buffer one thread takes every tile)
-            const int issuers = (shared_state || kStages < kIssuers * spt || (DUAL && nbuf < kIssuers)) ? 1 : kIssuers;
-            const int me = warp - 1;
-            int stage = 0; uint32_t phase = 0;
-            auto advance = [&](int n) {      // move n stages on (n >= 0)
-                stage += n;
-                while (stage >= kStages) { stage -= kStages; phase ^= 1u; }
-            };
-            advance(me * spt);
+            const int me = warp - 1, stage_lo = me * ring;
+            int stage = stage_lo; uint32_t phase = 0;
             int w_loads = resident ? 1 : 0;   // without shared state the resident weights are loaded exactly once
             int cur_n = -1;
             // patch mode with up to nine filter taps (3x3, 1x3 ...): the taps' window offsets live in registers
@@ -1113,7 +1123,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         tc_commit(bar_empty + 8 * stage);
                         TSB_CYC_ADD(cyc_commit);
                         st16 += stage16;
-                        if (++stage == kStages) { stage = 0; phase ^= 1u; st16 = base16; }
+                        if (++stage == stage_lo + ring) { stage = stage_lo; phase ^= 1u; st16 = base16 + (uint32_t)stage_lo * stage16; }
                     }
                 } else if (!SWAP && MODE == kModeRows) {
                     const int row_id = kp.d_segs.div(m_tile), seg = m_tile - row_id * kp.rows_segs;
@@ -1180,7 +1190,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     }
                     if (seg == kp.rows_segs - 1 || local == my_tiles - 1) {
                         tc_commit(bar_empty + 8 * stage);
-                        advance(1);
+                        if (++stage == stage_lo + ring) { stage = stage_lo; phase ^= 1u; }
                     }
                 } else {
                     // general mode: a stage holds kgroup K blocks; one wait, kgroup * BK/32 MMAs in a row, one commit
@@ -1223,7 +1233,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         TSB_CYC_ADD(cyc_commit);
                         w16 += (uint32_t)G * kWgt16;
                         st16 += stage16;
-                        if (++stage == kStages) { stage = 0; phase ^= 1u; st16 = base16; }
+                        if (++stage == stage_lo + ring) { stage = stage_lo; phase ^= 1u; st16 = base16 + (uint32_t)stage_lo * stage16; }
                     }
                 }
                 TSB_CYC_START;
@@ -1234,7 +1244,6 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     if (local + 1 < my_tiles) decode(local + 1, nm, nn);
                     if (nn != cur_n) tc_commit(bar_bfree);  // the resident weights may be replaced
                 }
-                advance((issuers - 1) * spt);             // skip the stages of the other issuers' tiles
                 if (me == 0) TSB_TRACE(local, 4);
             }
             if (me == 0) TSB_CYC_REPORT((my_tiles + issuers - 1) / issuers);
