@@ -49,16 +49,16 @@ struct tsb_conv_plan {
     tsb::tc::Config cfg;             // configuration with all shared memory given to the pipeline
     tsb::tc::Config cfg_alt;         // the other orientation (alt_valid): taken when the epilogue is pixel-major fp32 and no
     int alt_valid;                   // staged configuration fits
-    tsb::tc::Config cfg_stg[3];      // [1], [2]: configurations that set shared memory aside for the staged epilogue
-    int stg_valid[3];
+    tsb::tc::Config cfg_stg;         // configuration that sets shared memory aside for the staged epilogue
+    int stg_valid;
     int *status_word = nullptr;      // where the kernels report a wait that gave up, when not the workspace's first word
     size_t off_weights, off_stage, ws_bytes;
     // state bound by set_weights / run
     const int8_t *weights_oihw;      // direct kernel reads the caller's tensor
     const void *weights_ws;          // workspace the packed weights live in
-    CUtensorMap map_b, map_b_alt, map_b_stg[3];
-    const int8_t *map_a_ptr, *map_a_alt_ptr, *map_a_stg_ptr[3];
-    CUtensorMap map_a, map_a_alt, map_a_stg[3];
+    CUtensorMap map_b, map_b_alt, map_b_stg;
+    const int8_t *map_a_ptr, *map_a_alt_ptr, *map_a_stg_ptr;
+    CUtensorMap map_a, map_a_alt, map_a_stg;
     // tsb_conv2d_i8_run_projected: configuration and tensor maps of the last pair, reused while the four pointers, the
     // shortcut plan and the tile override stay the same
     struct {
@@ -207,12 +207,8 @@ int tsb_conv2d_i8_plan_create(const tsb_conv_desc *d, tsb_conv_plan **out) {
         p->cfg_alt = tc::choose_config(p->view, p->tune, sms, p->cfg.swap ? 0 : 1);
         // a forced orientation is final: the run-time choice by epilogue is only made between the library's own two plans
         p->alt_valid = p->cfg_alt.swap != p->cfg.swap && p->tune.orientation == 0;
-        for (int level = 1; level <= 2; ++level) {
-            p->cfg_stg[level] = tc::choose_config(p->view, p->tune, sms, -1, level);
-            const tc::Config &c = p->cfg_stg[level];
-            p->stg_valid[level] = c.staging == level && c.stages >= 2 && c.dyn_smem <= 227u * 1024u && (!p->view.rows || c.b_resident);
-            p->map_a_stg_ptr[level] = nullptr;
-        }
+        const tc::Config &c = p->cfg_stg = tc::choose_config(p->view, p->tune, sms, -1, true);
+        p->stg_valid = c.staging && c.stages >= 2 && c.dyn_smem <= 227u * 1024u && (!p->view.rows || c.b_resident);
         end = p->off_weights + align256(p->view.weight_bytes);
     }
     p->off_stage = end;
@@ -225,7 +221,8 @@ int tsb_conv2d_i8_plan_create(const tsb_conv_desc *d, tsb_conv_plan **out) {
     p->weights_ws = nullptr;
     p->map_a_ptr = nullptr;
     p->map_a_alt_ptr = nullptr;
-    if (p->kernel != TSB_KERNEL_TCGEN05) p->stg_valid[1] = p->stg_valid[2] = 0;
+    p->map_a_stg_ptr = nullptr;
+    if (p->kernel != TSB_KERNEL_TCGEN05) p->stg_valid = 0;
     *out = p;
     return TSB_OK;
 }
@@ -261,11 +258,10 @@ int tsb_conv2d_i8_plan_describe(const tsb_conv_plan *plan, char *text, size_t te
             len += snprintf(text + len, text_bytes - len, " | alt: ");
             if ((size_t)len < text_bytes) len += one(plan->cfg_alt, text + len, text_bytes - len);
         }
-        for (int level = 1; level <= 2; ++level)
-            if (plan->stg_valid[level] && len > 0 && (size_t)len < text_bytes) {
-                len += snprintf(text + len, text_bytes - len, " | staged%d: ", level);
-                if ((size_t)len < text_bytes) len += one(plan->cfg_stg[level], text + len, text_bytes - len);
-            }
+        if (plan->stg_valid && len > 0 && (size_t)len < text_bytes) {
+            len += snprintf(text + len, text_bytes - len, " | staged (%d): ", plan->cfg_stg.staging);
+            if ((size_t)len < text_bytes) len += one(plan->cfg_stg, text + len, text_bytes - len);
+        }
     }
     if (len < 0) return fail(TSB_ERR_INVALID_ARGUMENT, "plan_describe: formatting failed");
     return (size_t)len < text_bytes ? len : (int)text_bytes - 1;
@@ -292,11 +288,10 @@ int tsb_conv2d_i8_set_weights(tsb_conv_plan *plan, const int8_t *w_oihw, void *w
             st = tc::encode_weight_map(plan->view, plan->cfg_alt, wp, &plan->map_b_alt);
             if (st != TSB_OK) return st;
         }
-        for (int level = 1; level <= 2; ++level)
-            if (plan->stg_valid[level]) {
-                st = tc::encode_weight_map(plan->view, plan->cfg_stg[level], wp, &plan->map_b_stg[level]);
-                if (st != TSB_OK) return st;
-            }
+        if (plan->stg_valid) {
+            st = tc::encode_weight_map(plan->view, plan->cfg_stg, wp, &plan->map_b_stg);
+            if (st != TSB_OK) return st;
+        }
     }
     return TSB_OK;
 }
@@ -387,14 +382,13 @@ int tsb_conv2d_i8_run(tsb_conv_plan *plan, const int8_t *x, int x_layout, const 
     }
     // Outputs that can go through shared-memory tiles and tensor-map stores (int8 NHWC_PAD, pixel-major fp32 with or
     // without a residual) take the configuration that sets the tiles' shared memory aside.
-    const int level = tc::staging_level(plan->view, epi);
-    if (level != 0 && plan->stg_valid[level]) {
-        if (plan->map_a_stg_ptr[level] != x_tc) {
-            st = tc::encode_activation_map(plan->view, plan->cfg_stg[level], x_tc, &plan->map_a_stg[level]);
+    if (plan->stg_valid && tc::wants_staging(plan->view, epi)) {
+        if (plan->map_a_stg_ptr != x_tc) {
+            st = tc::encode_activation_map(plan->view, plan->cfg_stg, x_tc, &plan->map_a_stg);
             if (st != TSB_OK) return st;
-            plan->map_a_stg_ptr[level] = x_tc;
+            plan->map_a_stg_ptr = x_tc;
         }
-        return tc::launch_conv_tc(plan->view, plan->cfg_stg[level], plan->map_a_stg[level], plan->map_b_stg[level], x_tc, epi,
+        return tc::launch_conv_tc(plan->view, plan->cfg_stg, plan->map_a_stg, plan->map_b_stg, x_tc, epi,
                                   plan->status_word ? plan->status_word : static_cast<int *>(workspace), stream);
     }
     // Otherwise pixel-major fp32 tensors (a network's residuals and block outputs) are stored coalesced when a thread owns
@@ -448,11 +442,12 @@ static int run_pair(tsb_conv_plan *plan, const int8_t *x, tsb_conv_plan *shortcu
     const int8_t *wp = static_cast<const int8_t *>(workspace) + plan->off_weights;
     const int8_t *wp2 = static_cast<const int8_t *>(shortcut->weights_ws) + shortcut->off_weights;
     auto &pr = plan->pair;
-    const int tile_key = tile_channels + (concat ? 1000 : 0);      // the two modes never share a configuration
+    const bool staging = !concat || tc::wants_staging(plan->view, epi);
+    const int tile_key = tile_channels + (concat ? 1000 : 0) + (staging ? 2000 : 0);   // these never share a configuration
     if (pr.x != x || pr.x2 != x_shortcut || pr.w != wp || pr.w2 != wp2 || pr.shortcut != shortcut || pr.tile != tile_key ||
         memcmp(&pr.shortcut_desc, &shortcut->desc, sizeof(tsb_conv_desc)) != 0) {
         pr.x = nullptr;     // invalid until every map is encoded
-        pr.cfg = tc::choose_config_dual(plan->view, shortcut->view, sms, tile_channels, concat);
+        pr.cfg = tc::choose_config_dual(plan->view, shortcut->view, sms, tile_channels, concat, staging);
         if (pr.cfg.stages < 2 || pr.cfg.dyn_smem > 227u * 1024u) return fail(TSB_ERR_UNSUPPORTED, "run_projected: the pair does not fit shared memory");
         if ((st = tc::encode_activation_map(plan->view, pr.cfg, x, &pr.map_a)) != TSB_OK) return st;
         if ((st = tc::encode_weight_map(plan->view, pr.cfg, wp, &pr.map_b)) != TSB_OK) return st;
@@ -493,7 +488,8 @@ static const char *wait_name(int code) {
         case 4: return "epilogue: accumulator ready";
         case 5: return "producer: resident weight tile free";
         case 6: return "MMA issuer: resident weight tile loaded";
-        case 7: return "epilogue: staged residual tile loaded";
+        case 7: return "epilogue: staged tile ready";
+        case 8: return "epilogue copies: staged tile written";
         default: return "unknown wait";
     }
 }

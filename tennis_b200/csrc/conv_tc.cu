@@ -119,31 +119,34 @@ bool make_view(const ConvGeom &g, const Tuning &tune, View *view, const char **w
     return true;
 }
 
-int staging_level(const View &v, const EpiParams &epi) {
+bool wants_staging(const View &v, const EpiParams &epi) {
     const ConvGeom &g = v.real;
-    if (epi.out_acc) return 0;
+    if (epi.out_acc) return false;
     const bool per_sample = epi.nscales > 1 && epi.nscales == g.N && epi.group_len == (uint32_t)(g.O * g.OH * g.OW);
-    if (epi.out_i8 && !(epi.i8_nhwc && (epi.nscales == 1 || per_sample))) return 0;
-    if (epi.out_i8 && reinterpret_cast<uintptr_t>(epi.out_i8) % 16) return 0;
+    if (epi.out_i8 && !(epi.i8_nhwc && (epi.nscales == 1 || per_sample))) return false;
+    if (epi.out_i8 && reinterpret_cast<uintptr_t>(epi.out_i8) % 16) return false;
     const bool f32_tiles = (epi.out_f32 || epi.residual) && epi.f32_nhwc;
     if (f32_tiles) {
         // tensor maps over [pixels][O] fp32: rows must be whole 16-byte units, the tensors 16-byte aligned and distinct
-        if (g.O % 4 != 0 || (const void *)epi.residual == (const void *)epi.out_f32) return 0;
-        if ((reinterpret_cast<uintptr_t>(epi.out_f32) | reinterpret_cast<uintptr_t>(epi.residual)) % 16) return 0;
-        return 2;
+        if (g.O % 4 != 0 || (const void *)epi.residual == (const void *)epi.out_f32) return false;
+        if ((reinterpret_cast<uintptr_t>(epi.out_f32) | reinterpret_cast<uintptr_t>(epi.residual)) % 16) return false;
+        return true;
     }
     // fp32 NCHW output, or int8 NHWC_PAD alone: the direct paths (a thread's 32 int8 channels are one 32-byte sector,
     // which two 16-byte stores write as well as a tile store would)
-    return 0;
+    return false;
 }
 
-Config choose_config(const View &v, const Tuning &tune, int sm_count, int orientation, int staging) {
+// Shared memory of the staged epilogue: per quad `tiles` fp32 tiles and an int8 tile.
+static uint32_t staged_bytes(int tiles) { return tiles ? kQuads * ((uint32_t)tiles * kStageF32Bytes + kStageI8Bytes) : 0u; }
+
+// tiles: fp32 tiles per quad of the staged epilogue, 0: not staged
+static Config plan_config(const View &v, const Tuning &tune, int sm_count, int orientation, int tiles_per_quad) {
     const ConvGeom &g = v.g;
     Config c;
     c.bk = (g.Cp % 128 == 0) ? 128 : 64;
     const int64_t M = (int64_t)g.N * g.OH * g.OW;
-    const uint32_t stg_bytes = staging == 2 ? kQuads * (kStageF32Bytes + kStageI8Bytes) : (staging == 1 ? kQuads * kStageI8Bytes : 0u);
-    const uint32_t budget = kSmemBudget - stg_bytes;
+    const uint32_t stg_bytes = staged_bytes(tiles_per_quad), budget = kSmemBudget - stg_bytes;
     // An MMA instruction costs the same 128 cycles for any N up to 256, so N should be 256 whenever possible.
     // Normal orientation: 128 pixels on M, up to 256 output channels on N.  Swapped orientation: channels on M,
     // 256 (or 128) pixels on N -- it halves the MMA count of narrow layers but its epilogue (one channel per thread)
@@ -176,7 +179,7 @@ Config choose_config(const View &v, const Tuning &tune, int sm_count, int orient
         c.bn = g.O > 128 ? 256 : (g.O > 64 ? 128 : 64);
         // the staged block epilogue over plain [pixels][channels] tiles (the 1x1 expansions of residual blocks) measured 3-5 %
         // faster with four 128-channel accumulators, one tile per epilogue quad, than with two 256-channel ones
-        if (staging == 2 && v.a_tiled && c.bn == 256) c.bn = 128;
+        if (tiles_per_quad && v.a_tiled && c.bn == 256) c.bn = 128;
         const int m_tiles128 = (int)ceil_div64(M, kBM);
         // a narrower N tile when the wide one leaves most SMs idle or the last wave nearly empty
         while (c.bn > 64) {
@@ -242,7 +245,10 @@ Config choose_config(const View &v, const Tuning &tune, int sm_count, int orient
         c.bar_off = (uint32_t)c.stages * c.stage_bytes;
     }
     // the staged epilogue's tiles (1024-byte aligned for the 128B swizzle) sit between the pipeline and the barriers
-    c.staging = c.swap ? 0 : staging;
+    c.staging = c.swap ? 0 : tiles_per_quad;
+    // The more of a group's quads work on one tile, the closer together the CTA's copies lie in memory; but a quad needs a
+    // chunk of its own (32 channels), and the tiles of a deep K come too slowly for one group to wait for each in turn.
+    c.stg_groups = v.a_tiled ? (c.bn >= 128 ? 1 : 2) : (c.bn >= 128 ? 2 : 4);
     if (c.staging) {
         c.stg_off = (c.bar_off + 1023u) & ~1023u;
         c.bar_off = c.stg_off + stg_bytes;
@@ -251,6 +257,18 @@ Config choose_config(const View &v, const Tuning &tune, int sm_count, int orient
                             (c.patch ? 4 * (uint32_t)(g.KH * g.KW) : 0);   // epilogue tables, then patch mode's tap table
     c.dyn_smem = tables + 1024;  // slack to align the tiles to 1024 bytes
     return c;
+}
+
+// Two fp32 tiles per quad for plain [pixels][channels] tiles (1x1 layers, which the copies bound) as long as two K blocks are left in
+// flight, even where the weights then have to be streamed; one for filters of several taps, whose pipeline is worth more than
+// the second tile.  Measured, two tiles against one, residual + fp32 + int8, 64 images: 128 -> 512 at 28 x 28 46 / 55 us,
+// 256 -> 1024 at 14 x 14 26 / 34 us; 16 images, 3x3 64 -> 64 at 152 x 152 94 / 52 us, 128 -> 128 at 76 x 76 40 / 35 us.
+Config choose_config(const View &v, const Tuning &tune, int sm_count, int orientation, bool staging) {
+    if (staging && v.a_tiled) {
+        const Config two = plan_config(v, tune, sm_count, orientation, 2);
+        if (two.staging && two.stages >= 2) return two;
+    }
+    return plan_config(v, tune, sm_count, orientation, staging ? 1 : 0);
 }
 
 bool dual_supported(const View &v, const View &sc, const char **why) {
@@ -264,7 +282,7 @@ bool dual_supported(const View &v, const View &sc, const char **why) {
     return true;
 }
 
-Config choose_config_dual(const View &v, const View &sc, int sm_count, int bn, bool concat) {
+static Config plan_config_dual(const View &v, const View &sc, int sm_count, int bn, bool concat, int tiles_per_quad) {
     const ConvGeom &g = v.g, &s = sc.g;
     Config c;
     c.bk = (g.Cp % 128 == 0 && s.Cp % 128 == 0) ? 128 : 64;
@@ -280,8 +298,7 @@ Config choose_config_dual(const View &v, const View &sc, int sm_count, int bn, b
     c.num_n_tiles = ceil_div(g.O, c.ch);
     const int64_t tiles = (int64_t)c.num_m_tiles * c.num_n_tiles;
     c.grid = (int)(tiles < sm_count ? tiles : sm_count);
-    const uint32_t stg_bytes = kQuads * (kStageF32Bytes + kStageI8Bytes);
-    const uint32_t budget = kSmemBudget - stg_bytes;
+    const uint32_t stg_bytes = staged_bytes(tiles_per_quad), budget = kSmemBudget - stg_bytes;
     const uint32_t p_bytes = (uint32_t)c.pix * c.bk, w_bytes = (uint32_t)c.ch * c.bk;
     const uint32_t k1 = (uint32_t)g.KH * g.KW * (g.Cp / c.bk), k2 = (uint32_t)(s.Cp / c.bk);
     const uint32_t w_total = (k1 + k2) * w_bytes;
@@ -308,12 +325,22 @@ Config choose_config_dual(const View &v, const View &sc, int sm_count, int bn, b
         c.b_off = 0;
         c.bar_off = (uint32_t)c.stages * c.stage_bytes;
     }
-    c.staging = 2;
+    c.staging = tiles_per_quad;
+    c.stg_groups = 1;
     c.stg_off = (c.bar_off + 1023u) & ~1023u;
     c.bar_off = c.stg_off + stg_bytes;
     const uint32_t tables = ((c.bar_off + 8 * num_barriers(c.stages) + 8 + 15) & ~15u) + kMaxAccBufs * 2 * (uint32_t)c.bn * 4;
     c.dyn_smem = tables + 1024;
     return c;
+}
+
+// (Measured, two tiles per quad against one: 64 + 64 -> 256 at 56 x 56, 64 images, whose weights stay resident either way, 67 / 73 us;
+// where the second tile evicts them, 128 + 256 -> 512 at 28 x 28 46 / 44 us and 256 + 512 -> 1024 at 14 x 14 33 / 28 us.)
+Config choose_config_dual(const View &v, const View &sc, int sm_count, int bn, bool concat, bool staging) {
+    const Config one = plan_config_dual(v, sc, sm_count, bn, concat, staging ? 1 : 0);
+    if (!staging) return one;
+    const Config two = plan_config_dual(v, sc, sm_count, bn, concat, 2);
+    return two.b_resident == one.b_resident && two.stages >= 2 ? two : one;
 }
 
 int encode_weight_map(const View &v, const Config &cfg, const int8_t *w_packed, CUtensorMap *map) {
@@ -465,7 +492,7 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
         const bool i8_ok = !epi.out_i8 || (epi.i8_nhwc && reinterpret_cast<uintptr_t>(epi.out_i8) % 16 == 0 &&
                                            (epi.nscales == 1 || (epi.nscales == g.N && epi.group_len == (uint32_t)(g.O * g.OH * g.OW))));
         const bool f32_ok = !epi.out_f32 || (epi.f32_nhwc && reinterpret_cast<uintptr_t>(epi.out_f32) % 16 == 0);
-        if (epi.out_acc || epi.residual || !i8_ok || !f32_ok || g.O % 4 != 0 || cfg.swap || cfg.patch || v.rows || v.fold || cfg.staging != 2)
+        if (epi.out_acc || epi.residual || !i8_ok || !f32_ok || g.O % 4 != 0 || cfg.swap || cfg.patch || v.rows || v.fold || (!cfg.staging && dual->dq))
             return fail(TSB_ERR_UNSUPPORTED, "projected shortcut: needs pixel-major fp32 / NHWC_PAD int8 outputs, no residual tensor, O %% 4 == 0");
     }
     KernelParams kp;
@@ -543,12 +570,13 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
     // like the pixel tile of the load mode (a run of pixels, a run inside one output row, or an 8 x 16 block).
     CUtensorMap map_of = map_b, map_oi = map_b;
     kp.stg_off = cfg.stg_off;
-    kp.stg_f32 = cfg.staging == 2 ? 1 : 0;
+    kp.stg_tiles = cfg.staging;
+    kp.stg_groups = cfg.stg_groups;
     // (a projection needs the staged epilogue, whose fp32 tile receives its result; a concatenation takes whatever epilogue
     // its outputs would take in a plain run -- int8 alone goes out through the direct path, which is faster for it)
     const bool dual_concat = dual && dual->dq == nullptr;
-    const int want_staging = (dual && !dual_concat) ? 2 : (cfg.swap ? 0 : staging_level(v, epi));
-    if (want_staging != 0 && cfg.staging >= want_staging && load_driver() == TSB_OK) {
+    const bool want_staging = (dual && !dual_concat) || wants_staging(v, epi);
+    if (want_staging && cfg.staging && load_driver() == TSB_OK) {
         const ConvGeom &r = v.real;
         auto encode = [&](CUtensorMap *map, const void *ptr, bool is_f32, uint64_t channels) -> bool {
             const uint64_t es = is_f32 ? 4 : 1;
@@ -582,14 +610,13 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
         if (epi.out_f32) ok_maps = ok_maps && encode(&map_of, epi.out_f32, true, (uint64_t)r.O);
         if (epi.out_i8) ok_maps = ok_maps && encode(&map_oi, epi.out_i8, false, (uint64_t)epi.out_cp);
         if (ok_maps) {
-            epi_mode = kEpiStaged;
+            epi_mode = epi.res_after ? kEpiStagedAfter : kEpiStaged;
             kp.res_prefetch = 0;
-            kp.stg_f32 = cfg.staging == 2 ? 1 : 0;
         }
     }
     if (dual) {
-        if (!dual_concat && epi_mode != kEpiStaged) return fail(TSB_ERR_UNSUPPORTED, "projected shortcut: the output tensor maps could not be encoded");
-        if (dual_concat && epi_mode != kEpiStaged && epi_mode != kEpiI8Nhwc)
+        if (!dual_concat && !is_staged(epi_mode)) return fail(TSB_ERR_UNSUPPORTED, "projected shortcut: the output tensor maps could not be encoded");
+        if (dual_concat && !is_staged(epi_mode) && epi_mode != kEpiI8Nhwc)
             return fail(TSB_ERR_UNSUPPORTED, "concatenated input: outputs must be pixel-major fp32 and / or NHWC_PAD int8");
         const ConvGeom &s = dual->view->g;
         DualParams dp;

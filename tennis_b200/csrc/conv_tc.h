@@ -50,7 +50,8 @@ struct Config {
     int kgroup = 1;                   // K blocks per pipeline stage (im2col / tiled loads; 1 in patch and raw-row mode)
     uint32_t unit_bytes = 0;          // one K block of a stage
     uint32_t stage_bytes = 0, b_off = 0, bar_off = 0, dyn_smem = 0;
-    int staging = 0;                  // shared memory set aside for the staged epilogue: 0 none, 1 int8 tiles, 2 fp32 + int8 tiles
+    int staging = 0;                  // fp32 tiles per quad that shared memory is set aside for (staged epilogue): 0, 1 or 2
+    int stg_groups = 4;               // groups of epilogue warps in the staged class
     uint32_t stg_off = 0;
 };
 
@@ -66,12 +67,11 @@ struct Tuning {
 bool make_view(const ConvGeom &g, const Tuning &tune, View *view, const char **why);
 // orientation: -1 = by heuristic (or tune.orientation), 0 = normal, 1 = swapped (any number of output channels, 128
 // per channel tile)
-// staging: shared memory to set aside for the staged epilogue (see Config::staging); only normal-orientation
+// staging: set shared memory aside for the staged epilogue (see Config::staging); only normal-orientation
 // configurations use it
-Config choose_config(const View &v, const Tuning &tune, int sm_count, int orientation, int staging = 0);
-// Which staged epilogue these outputs can take with this view: 0 none (direct stores), 1 int8 NHWC_PAD tile only,
-// 2 pixel-major fp32 residual / output (and int8) tiles.
-int staging_level(const View &v, const EpiParams &epi);
+Config choose_config(const View &v, const Tuning &tune, int sm_count, int orientation, bool staging = false);
+// Whether these outputs can take the staged epilogue: pixel-major fp32 residual and / or output, with or without int8 NHWC_PAD.
+bool wants_staging(const View &v, const EpiParams &epi);
 // w_packed: [O][KH][KW][Cp] int8 of the view's geometry
 int encode_weight_map(const View &v, const Config &cfg, const int8_t *w_packed, CUtensorMap *map);
 // x: the staged activations (NHWC_PAD or folded), 16-byte aligned
@@ -97,8 +97,9 @@ struct DualArgs {
 };
 // whether `shortcut` can run inside the kernel of `v`; *why names the reason when it cannot
 bool dual_supported(const View &v, const View &shortcut, const char **why);
-// one configuration for the pair: common K block, both weight tiles resident when they fit; bn: 0 = by output channels
-Config choose_config_dual(const View &v, const View &shortcut, int sm_count, int bn, bool concat = false);
+// one configuration for the pair: common K block, both weight tiles resident when they fit; bn: 0 = by output channels;
+// staging: with the staged epilogue's tiles (always for a projection; for a concatenation as its outputs want)
+Config choose_config_dual(const View &v, const View &shortcut, int sm_count, int bn, bool concat, bool staging);
 // x_staged: the activations the map_a was encoded for (read directly in raw-row mode)
 int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, const CUtensorMap &map_b,
                    const int8_t *x_staged, const EpiParams &epi, int *status_word, cudaStream_t stream,

@@ -35,10 +35,10 @@ namespace tc {
 constexpr int kBM = 128;
 constexpr int kIssuers = 2;                              // warps that issue MMAs, on alternate tiles
 constexpr int kEpiWarp0 = 1 + kIssuers;                  // first epilogue warp
-constexpr int kEpiThreads = 512;
-constexpr int kThreads = 32 * kEpiWarp0 + kEpiThreads;   // producer warp, issuer warps, sixteen epilogue warps
+constexpr int kEpiThreads = 512;                         // sixteen epilogue warps
+constexpr int kCopyWarp0 = kEpiWarp0 + kEpiThreads / 32; // staged epilogue: the first of its four copy warps
 constexpr int kMaxAccBufs = 4;                           // accumulator buffers in tensor memory (512 columns / BN, at most 4)
-constexpr uint32_t kSmemBudget = 200 * 1024;  // stages; the rest holds barriers and epilogue tables
+constexpr uint32_t kSmemBudget = 216 * 1024;  // stages and staged tiles; the rest of the 227 KB holds barriers and epilogue tables
 
 // ---------------------------------------------------------------------------------------------------------
 // PTX wrappers
@@ -113,17 +113,6 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 // generic-proxy writes to shared memory become visible to the async proxy (TMA) of this CTA
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// named barrier over `threads` threads that also ORs a predicate over them
-__device__ __forceinline__ bool bar_or(int id, int threads, bool pred) {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, %2, %3, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(r) : "r"((uint32_t)pred), "r"(id), "r"(threads) : "memory");
-    return r != 0;
-}
 __device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c, int w,
                                                    int h, int n, uint16_t off_w, uint16_t off_h) {
     asm volatile(
@@ -135,6 +124,11 @@ __device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const CUtensorM
 // Brings a box of a tensor into L2 without a destination in shared memory (no barrier, nothing to wait for).
 __device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap *map, int x, int y) {
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+
+// Brings a tensor map (a kernel parameter) into the copy engine's descriptor cache.
+__device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t cols) {
@@ -260,6 +254,10 @@ constexpr int kEpiF32Nchw = 1;   // fp32 NCHW output only (the operator's own ou
 constexpr int kEpiI8Nhwc = 2;    // requantized int8 NHWC_PAD output only, half-away rounding, one scale per sample
 constexpr int kEpiNhwc = 3;      // fp32 [N][P][O] residual in and/or fp32 [N][P][O] out and/or int8 NHWC_PAD out (swapped orientation)
 constexpr int kEpiStaged = 4;    // the same outputs through shared-memory tiles and tensor-map loads / stores (normal orientation)
+constexpr int kEpiStagedAfter = 5;   // ... with the residual added after the activation
+__host__ __device__ constexpr bool is_staged(int epi) { return epi == kEpiStaged || epi == kEpiStagedAfter; }
+// producer warp, issuer warps, sixteen epilogue warps and, in the staged class, four copy warps
+__host__ __device__ constexpr int cta_threads(int epi) { return 32 * (kCopyWarp0 + (is_staged(epi) ? 4 : 0)); }
 constexpr uint32_t kStageF32Bytes = kBM * 32 * 4;   // one staged fp32 tile: 128 pixels x 32 channels, 128-byte rows, swizzle 128B
 constexpr uint32_t kStageI8Bytes = kBM * 32;        // one staged int8 tile: 128 pixels x 32 channels, 32-byte rows
 constexpr int kQuads = 4;                           // the sixteen epilogue warps form four quads of one warp per lane quarter
@@ -404,22 +402,33 @@ __device__ __forceinline__ bool store_i8_nhwc_t(const int (&v)[W], const float *
 }
 
 // Block-output epilogue of a residual network: v = act(dq*acc + bias + residual); fp32 copy for the next residual and
-// int8 copy for the next convolution, each optional.  The thread's 32 channels of residual come from its row of a shared-memory tile
-// that a tensor-map load filled (128-byte rows, 128B swizzle: 16-byte chunk i of row r sits at chunk i ^ (r & 7)), the
+// int8 copy for the next convolution, each optional.  The thread's 32 channels of residual come from its row of a shared-memory
+// tile that a tensor-map load filled (128-byte rows, 128B swizzle: 16-byte chunk i of row r sits at chunk i ^ (r & 7)), the
 // fp32 results go back into the same places and the int8 results into the thread's 32-byte row of a second tile; tensor-
 // map stores carry both tiles to global memory.  No global address arithmetic, every shared-memory access 16 bytes wide.
+// r_row: shared-memory address of the row, its swizzle key folded in, so that chunk i is at r_row ^ (i * 16).
+__device__ __forceinline__ float4 lds128(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts128(uint32_t addr, float4 v) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// Returns false when an int8 value needs the exact conversion (NaN, beyond the int32 range).  q: the packed int8 results.
 template <int ACT, bool EVEN, bool AFTER>
 __device__ __forceinline__ bool staged_chunk_t(const int (&v)[32], const float *__restrict__ dq, const float *__restrict__ bias,
-                                               float leaky, float4 *__restrict__ r_row, int key, bool has_res, bool has_f32,
-                                               int4 *__restrict__ q_row, bool has_i8, float rs) {
-    uint32_t q[8];
+                                               float leaky, uint32_t r_row, bool has_res, bool has_i8, float rs, uint32_t (&q)[8]) {
     float worst = 0.0f;
 #pragma unroll
     for (int j4 = 0; j4 < 8; ++j4) {
         const float4 d4 = *reinterpret_cast<const float4 *>(dq + 4 * j4);
         const float4 b4 = *reinterpret_cast<const float4 *>(bias + 4 * j4);
         float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (has_res) r4 = r_row[j4 ^ key];
+        if (has_res) r4 = lds128(r_row ^ (uint32_t)(j4 * 16));
         float f[4];
         const float dd[4] = {d4.x, d4.y, d4.z, d4.w}, bb[4] = {b4.x, b4.y, b4.z, b4.w}, rr[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
@@ -433,19 +442,14 @@ __device__ __forceinline__ bool staged_chunk_t(const int (&v)[32], const float *
             if (AFTER) t = __fadd_rn(t, rr[k]);
             f[k] = t;
         }
-        if (has_f32) r_row[j4 ^ key] = make_float4(f[0], f[1], f[2], f[3]);
+        sts128(r_row ^ (uint32_t)(j4 * 16), make_float4(f[0], f[1], f[2], f[3]));
         if (has_i8) {
             const float t0 = __fmul_rn(f[0], rs), t1 = __fmul_rn(f[1], rs), t2 = __fmul_rn(f[2], rs), t3 = __fmul_rn(f[3], rs);
             worst = max3_nan(max3_nan(worst, fabsf(t0), fabsf(t1)), fabsf(t2), fabsf(t3));
             q[j4] = pack_sat_s8(round_s32<EVEN>(t0), round_s32<EVEN>(t1), round_s32<EVEN>(t2), round_s32<EVEN>(t3));
         }
     }
-    if (has_i8) {
-        if (!(worst < 2147483648.0f)) return false;
-        q_row[0] = make_int4(q[0], q[1], q[2], q[3]);
-        q_row[1] = make_int4(q[4], q[5], q[6], q[7]);
-    }
-    return true;
+    return worst < 2147483648.0f;
 }
 
 // ---- fast paths, swapped orientation: the thread owns one CHANNEL (its lane) and 32 consecutive pixels; dq and bias
@@ -678,8 +682,9 @@ struct KernelParams {
     int b_resident;        // all K blocks of this CTA's weight tile stay in shared memory; only activations stream
     uint32_t b_off;        // offset of the resident weights
     uint32_t bar_off;      // offset of the mbarriers; tensor-memory slot, abort flag and epilogue tables follow
-    uint32_t stg_off;      // staged epilogue: offset of the four quads' tiles (1024-aligned); per quad an fp32 tile (when
-    int stg_f32;           // stg_f32) followed by an int8 tile
+    uint32_t stg_off;      // staged epilogue: offset of its tiles (1024-aligned): the quads' fp32 tiles, then one int8 tile per quad
+    int stg_tiles;         // fp32 tiles per quad: 1 or 2
+    int stg_groups;        // groups of epilogue warps, each on its own tile (1, 2 or 4; fewer where the CTA has fewer tiles)
     // raw-row mode (rows_segs > 0): a tile is up to 128 consecutive pixels of ONE output row; per filter row the
     // producer copies the staged bytes under those pixels once, and the MMA reads them through a sliding descriptor
     int rows_segs;         // tiles per output row (0: mode off)
@@ -762,8 +767,9 @@ struct NoDual {};
 constexpr int kMaxStages = 24;
 constexpr uint32_t kMaxDynamicSmem = 227 * 1024;
 
-// barriers: full[stages], empty[stages], tmem_full[4], tmem_empty[4], b_full, b_free, staged_residual[4]
-__host__ __device__ constexpr uint32_t num_barriers(int stages) { return 2u * (uint32_t)stages + 2u * kMaxAccBufs + 2u + 4u; }
+// barriers, in this order: full[stages], empty[stages], tmem_full[4], tmem_empty[4], b_full, b_free, and for the staged
+// epilogue's tiles ready[4 quads][2], full[4][2], int8_free[4]
+__host__ __device__ constexpr uint32_t num_barriers(int stages) { return 2u * (uint32_t)stages + 2u * kMaxAccBufs + 2u + 5u * kQuads; }
 
 // PIX pixels x CH channels per tile.  Normal orientation: the pixel tile is the MMA's A operand (M = 128 pixels), the
 // weight tile its B operand (N = BN channels).  Swapped orientation: the weight tile is A (M = 128 channels, rows
@@ -773,14 +779,14 @@ __host__ __device__ constexpr uint32_t num_barriers(int stages) { return 2u * (u
 // MODE: how activations reach shared memory -- kModeGeneral (im2col or plain 2-D tile loads), kModeRows (raw-row), kModePatch.
 // A compile-time parameter: the role loops of each mode stay short and keep their registers.
 template <int BN, int BK, bool SWAP, int MODE, int EPI, bool DUAL>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(cta_threads(EPI), 1)
 conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_of,
                   const __grid_constant__ CUtensorMap map_oi, const __grid_constant__ KernelParams kp,
                   const __grid_constant__ EpiParams epi,
                   const __grid_constant__ std::conditional_t<DUAL, DualParams, NoDual> dual) {
     static_assert(!DUAL || (!SWAP && MODE == kModeGeneral), "projected-shortcut kernels: normal orientation, general mode");
-    static_assert(SWAP ? EPI != kEpiStaged : EPI != kEpiNhwc, "pixel-major fp32 tensors: staged tiles where a thread owns a pixel");
+    static_assert(SWAP ? !is_staged(EPI) : EPI != kEpiNhwc, "pixel-major fp32 tensors: staged tiles where a thread owns a pixel");
     constexpr int PIX = SWAP ? BN : kBM;      // pixels per tile
     constexpr int CH = SWAP ? kBM : BN;       // output channels per tile
     constexpr uint32_t kPixBytes = PIX * BK, kWgtBytes = CH * BK;
@@ -798,7 +804,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const uint32_t bar_tempty = bar_tfull + 8 * kMaxAccBufs;
     const uint32_t bar_bfull = bar_tempty + 8 * kMaxAccBufs;
     const uint32_t bar_bfree = bar_bfull + 8;
-    const uint32_t bar_stg = bar_bfree + 8;     // one per epilogue quad: a staged residual tile has landed
+    const uint32_t bar_stg = bar_bfree + 8;     // the staged epilogue's
     const uint32_t slot_off = kp.bar_off + 8 * num_barriers(kStages);
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(base_ptr + slot_off);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(base_ptr + slot_off + 4);
@@ -823,6 +829,8 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     // tiles -- a CTA with a single tile puts all sixteen epilogue warps on it.
     // (a projected-shortcut tile holds two accumulators: buffers 2a and 2a+1 of logical buffer a)
     const int nbuf = DUAL ? ((kBufs >= 4 && my_tiles >= 2) ? 2 : 1) : (my_tiles >= 4 && kBufs >= 4 ? 4 : (my_tiles >= 2 ? 2 : 1));
+    // Epilogue groups: one per buffer, each on its own tile; in the staged class as many as the configuration says.
+    const int groups = is_staged(EPI) ? min(kp.stg_groups, nbuf) : nbuf;
     auto decode = [&](int i, int &m_tile, int &n_tile) {   // m_tile: pixel tile, n_tile: channel tile
         if (kp.b_resident) {
             const int t = tile_lo + i;
@@ -833,14 +841,23 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
     };
 
-    if (threadIdx.x == 0) {
-        TSB_TRACE(0, 7);
-        for (int s = 0; s < kStages; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
-        for (int a = 0; a < kMaxAccBufs; ++a) { mbar_init(bar_tfull + 8 * a, 1); mbar_init(bar_tempty + 8 * a, kEpiThreads / nbuf); }
-        mbar_init(bar_bfull, 1);
-        mbar_init(bar_bfree, 1);
-        for (int q = 0; q < kQuads; ++q) mbar_init(bar_stg + 8 * q, 1);
-        *abort_flag = 0;
+    if (threadIdx.x == 0) TSB_TRACE(0, 7);
+    if (warp == 0) {
+        // one barrier per lane and step (a single thread takes 0.3 us for the eighty of them); the descriptors' first fetch
+        // overlaps the wait for the previous kernel
+        for (int i = lane; i < (int)num_barriers(kStages); i += 32) {
+            const int t = i - 2 * kStages;                                            // full, empty: one arrival each
+            const bool tempty = t >= kMaxAccBufs && t < 2 * kMaxAccBufs;
+            const int stg = t - (2 * kMaxAccBufs + 2);                                // staged tiles: ready, full, int8 free
+            const bool full = stg >= 2 * kQuads && stg < 4 * kQuads;
+            mbar_init(bar_full + 8 * i, tempty ? kEpiThreads / groups : (full ? 4 : 1));
+        }
+        if (lane == 0) {
+            *abort_flag = 0;
+            if (MODE != kModeRows) prefetch_tensormap(&map_a);
+            prefetch_tensormap(&map_b);
+            if constexpr (DUAL) { prefetch_tensormap(&dual.map_a2); prefetch_tensormap(&dual.map_b2); }
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -1248,14 +1265,102 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
             if (me == 0) TSB_CYC_REPORT((my_tiles + issuers - 1) / issuers);
         }
+    } else if (is_staged(EPI) && warp >= kCopyWarp0) {
+        // ------------------------------------------------------------------ staged epilogue: copies
+        // One thread per quad moves the quad's tiles, so that the arithmetic warps neither issue copies nor wait for them.  A tile
+        // is loaded (residual), worked on and stored; with two tiles per quad the store of one chunk and the load of the next
+        // but one run under the arithmetic of the chunk between them.  What is left is what the copies themselves cost: tensor-map
+        // copies alone (a box in, a box out, 412 MB) run at 5.3-5.5 TB/s here, 64 -> 256 channels at 56 x 56 with a residual (474 MB,
+        // 64 images) at 4.8.  (With the quad's first warp issuing the copies and one
+        // tile, a chunk of 128 pixels x 32 channels took 7700 cycles, of which the arithmetic was 1900, waiting for the residual
+        // 1260, issuing copies 550, waiting until a store had read the tile 700, barriers and the rest 1200.)
+        if (lane == 0) {
+            const int quad = warp - kCopyWarp0, parts = kQuads / groups, group = quad / parts, part = quad % parts;
+            const int tiles = kp.stg_tiles;
+            const bool has_res = epi.residual != nullptr, has_f32 = epi.out_f32 != nullptr, has_i8 = epi.out_i8 != nullptr;
+            const uint32_t f_tile = base + kp.stg_off + (uint32_t)(quad * tiles) * kStageF32Bytes;
+            const uint32_t q_tile = base + kp.stg_off + (uint32_t)(kQuads * tiles) * kStageF32Bytes + (uint32_t)quad * kStageI8Bytes;
+            const uint32_t ready = bar_stg + 8 * (quad * 2), full = bar_stg + 8 * (2 * kQuads + quad * 2), q_free = bar_stg + 8 * (4 * kQuads + quad);
+            if (has_res) prefetch_tensormap(&map_r);
+            if (has_f32) prefetch_tensormap(&map_of);
+            if (has_i8) prefetch_tensormap(&map_oi);
+            // a walk over the quad's chunks: tile coordinates (innermost: the channel) and the position in the channel tile
+            struct Walk { int local, c, nchunks, o_base, c1, c2, c3; };
+            auto enter = [&](Walk &w) {            // at the first chunk of tile w.local
+                if (w.local >= my_tiles) return;
+                int m_tile, n_tile;
+                decode(w.local, m_tile, n_tile);
+                w.o_base = n_tile * CH;
+                const int ch_end = min(w.o_base + BN, max(epi.O, has_i8 ? epi.out_cp : 0));
+                w.nchunks = ch_end > w.o_base ? (ch_end - w.o_base + 31) >> 5 : 0;
+                w.c = part;
+                w.c1 = m_tile * PIX; w.c2 = 0; w.c3 = 0;                          // general: [pixel][channel]
+                if (MODE == kModeRows) {                                        // [image row][ow][channel]
+                    const int row_id = kp.d_segs.div(m_tile);
+                    w.c1 = (m_tile - row_id * kp.rows_segs) * PIX; w.c2 = row_id;
+                }
+                if (MODE == kModePatch) {                                       // [image][oh][ow][channel]
+                    const int p_img = kp.d_tiles_hw.div(m_tile), p_rem = m_tile - p_img * kp.patch_tiles_hw;
+                    const int p_r = kp.d_tiles_w.div(p_rem), p_c = p_rem - p_r * kp.patch_tiles_w;
+                    w.c1 = p_c * 8; w.c2 = p_r * (PIX / 8); w.c3 = p_img;
+                }
+            };
+            auto settle = [&](Walk &w) {           // skip tiles in which this quad has no chunk (left)
+                while (w.local < my_tiles && w.c >= w.nchunks) { w.local += groups; enter(w); }
+            };
+            // makes tile t ready for the chunk at w and moves w on
+            auto load = [&](Walk &w, int t) {
+                if (w.local >= my_tiles) return;
+                const int ch = w.o_base + w.c * 32;
+                const uint32_t bar = ready + 8 * t;
+                if (has_res && ch < epi.O) {
+                    const uint32_t dst = f_tile + (uint32_t)t * kStageF32Bytes;
+                    mbar_arrive_expect_tx(bar, kStageF32Bytes);
+                    if (MODE == kModePatch) tma_load_4d(dst, &map_r, bar, ch, w.c1, w.c2, w.c3);
+                    else if (MODE == kModeRows) tma_load_3d(dst, &map_r, bar, ch, w.c1, w.c2);
+                    else tma_load_2d(dst, &map_r, bar, ch, w.c1);
+                } else {
+                    mbar_arrive(bar);
+                }
+                w.c += parts;
+                settle(w);
+            };
+            auto store = [&](const CUtensorMap *map, uint32_t src, const Walk &w, int ch) {
+                if (MODE == kModePatch) tma_store_4d(map, src, ch, w.c1, w.c2, w.c3);
+                else if (MODE == kModeRows) tma_store_3d(map, src, ch, w.c1, w.c2);
+                else tma_store_2d(map, src, ch, w.c1);
+            };
+            Walk in, out;
+            in.local = group; in.c = in.nchunks = in.o_base = in.c1 = in.c2 = in.c3 = 0;
+            enter(in);
+            settle(in);
+            out = in;
+            for (int t = 0; t < tiles; ++t) load(in, t);
+            for (int i = 0; out.local < my_tiles; ++i) {
+                const int t = i & (tiles - 1);
+                if (!mbar_wait(full + 8 * t, (uint32_t)(tiles == 2 ? i >> 1 : i) & 1u, abort_flag)) {
+                    if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 8); }
+                    break;
+                }
+                const int ch = out.o_base + out.c * 32;
+                if (has_f32 && ch < epi.O) store(&map_of, f_tile + (uint32_t)t * kStageF32Bytes, out, ch);
+                if (has_i8) store(&map_oi, q_tile, out, ch);
+                bulk_commit();
+                bulk_wait_read();                                    // the tiles may be overwritten
+                if (has_i8) mbar_arrive(q_free);
+                load(in, t);
+                out.c += parts;
+                settle(out);
+            }
+        }
     } else {
-        // ------------------------------------------------------------------ epilogue (the last sixteen warps)
+        // ------------------------------------------------------------------ epilogue (sixteen warps)
         // A warp may read only the 32 tensor-memory lanes of its quarter (warp id mod 4); four warps share a
         // quarter and split the tile's columns between them in chunks of 32.
-        // The sixteen warps form nbuf groups (of four, eight or all sixteen warps); group g owns accumulator buffer g and
-        // takes the tiles local = g, g + nbuf, ...  One tile's epilogue is a chain of latencies (barrier, tensor-memory
+        // The sixteen warps form groups (of four, eight or all sixteen warps); group g takes the tiles local = g, g + groups, ...
+        // One tile's epilogue is a chain of latencies (barrier, tensor-memory
         // load, arithmetic, stores); with the groups on different tiles those chains overlap.
-        const int group_warps = 16 / nbuf;                       // 4, 8 or 16
+        const int group_warps = 16 / groups;                       // 4, 8 or 16
         const int group_threads = 32 * group_warps;
         const int parts = group_warps / 4;                       // warps of a group per lane quarter: 1, 2 or 4
         const int quarter = warp & 3;
@@ -1266,16 +1371,16 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         constexpr int kChunks = BN / 32;
         constexpr int CW = 32;                   // normal orientation: columns a warp takes per step
         const int act = epi.activation;
-        uint32_t stg_phase[1] = {0u};            // staged epilogue: phase of this quad's residual barrier
+        int stg_count = 0;                       // staged epilogue: chunks this quad has worked through
         int table_n = -1;                        // channel tile this group's scale / bias table holds
-        for (int local = group; local < my_tiles; local += nbuf) {
-            const int acc = group;
+        for (int local = group; local < my_tiles; local += groups) {
+            const int acc = local & (nbuf - 1);
             const uint32_t acc_phase = (uint32_t)(local / nbuf) & 1u;
             int m_tile, n_tile;
             decode(local, m_tile, n_tile);
             const int o_base = n_tile * CH;
-            const int slot = DUAL ? 2 * acc : acc;          // first accumulator buffer (and table) of this tile
-            float *t_dq = table + slot * 2 * BN, *t_bias = t_dq + BN;
+            const int slot = DUAL ? 2 * acc : acc;          // first accumulator buffer of this tile
+            float *t_dq = table + (DUAL ? 2 * group : group) * 2 * BN, *t_bias = t_dq + BN;
             if (!SWAP && n_tile != table_n) {
                 // this group's table of per-channel scales and biases: rebuilt only when the channel tile changes (never, for
                 // layers of at most BN channels), between two barriers of the group
@@ -1323,137 +1428,84 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 }
                 const int img = live ? kp.d_P.div(m) : 0;
                 const int p = live ? m - img * kp.P : 0;
-                if constexpr (EPI == kEpiStaged) {
-                    // ---- staged epilogue: residual in by tensor-map load, fp32 / int8 tiles out by tensor-map stores.
+                if constexpr (is_staged(EPI)) {
+                    // ---- staged epilogue, the arithmetic: residual tile -> result tiles, all in shared memory.
                     // A quad (the four warps of this group that share `part`, one per lane quarter = the tile's 128
-                    // pixels) owns one fp32 tile and one int8 tile in shared memory and works through its 32-channel
-                    // chunks; the warp of lane quarter 0 issues the quad's copies.
+                    // pixels) works through its 32-channel chunks; its copy warp brings the residual tiles and carries the
+                    // result tiles off (below).  The warps of a quad do not wait for each other.
                     const int quad = group * parts + part;
-                    const int bar_id = 5 + quad;                                   // named barriers 1..4 belong to the groups
-                    const uint32_t stg = base + kp.stg_off + (uint32_t)quad * ((kp.stg_f32 ? kStageF32Bytes : 0u) + kStageI8Bytes);
-                    float4 *r_tile = reinterpret_cast<float4 *>(base_ptr + (stg - base));
-                    int4 *q_tile = reinterpret_cast<int4 *>(base_ptr + (stg - base) + (kp.stg_f32 ? kStageF32Bytes : 0u));
-                    const uint32_t q_addr = stg + (kp.stg_f32 ? kStageF32Bytes : 0u);
-                    const uint32_t rbar = bar_stg + 8 * quad;
-                    const bool leader = quarter == 0 && lane == 0;
-                    const bool has_res = epi.residual != nullptr, has_f32 = epi.out_f32 != nullptr, has_i8 = epi.out_i8 != nullptr;
-                    // tile coordinates of the three tensor maps (innermost coordinate: the channel)
-                    int c1 = m_tile * PIX, c2 = 0, c3 = 0;                          // general: [pixel][channel]
-                    if (MODE == kModeRows) {                                      // [image row][ow][channel]
-                        const int row_id = kp.d_segs.div(m_tile);
-                        c1 = (m_tile - row_id * kp.rows_segs) * PIX; c2 = row_id;
-                    }
-                    if (MODE == kModePatch) {                                     // [image][oh][ow][channel]
-                        const int p_img = kp.d_tiles_hw.div(m_tile), p_rem = m_tile - p_img * kp.patch_tiles_hw;
-                        const int p_r = kp.d_tiles_w.div(p_rem), p_c = p_rem - p_r * kp.patch_tiles_w;
-                        c1 = p_c * 8; c2 = p_r * (PIX / 8); c3 = p_img;
-                    }
-                    auto load_res = [&](int ch) {
-                        mbar_arrive_expect_tx(rbar, kStageF32Bytes);
-                        if (MODE == kModePatch) tma_load_4d(stg, &map_r, rbar, ch, c1, c2, c3);
-                        else if (MODE == kModeRows) tma_load_3d(stg, &map_r, rbar, ch, c1, c2);
-                        else tma_load_2d(stg, &map_r, rbar, ch, c1);
-                    };
-                    auto store_tile = [&](const CUtensorMap *map, uint32_t src, int ch) {
-                        if (MODE == kModePatch) tma_store_4d(map, src, ch, c1, c2, c3);
-                        else if (MODE == kModeRows) tma_store_3d(map, src, ch, c1, c2);
-                        else tma_store_2d(map, src, ch, c1);
-                    };
+                    const uint32_t q_row = base + kp.stg_off + (uint32_t)(kQuads * kp.stg_tiles) * kStageF32Bytes + (uint32_t)quad * kStageI8Bytes + (uint32_t)row * 32u;
+                    const bool has_res = epi.residual != nullptr, has_i8 = epi.out_i8 != nullptr;
                     // channels this tile has to cover: the real ones, and for an int8 output its zero padding as well
                     const int ch_end = min(o_base + BN, max(epi.O, has_i8 ? epi.out_cp : 0));
                     const int nchunks = ch_end > o_base ? (ch_end - o_base + 31) >> 5 : 0;
                     const float rs = epi.nscales == 1 ? epi.rq_scales[0] : epi.rq_scales[min(img, epi.nscales - 1)];
-                    const int key = row & 7;
-                    float4 *r_row = r_tile + row * 8;
-                    int4 *q_row = q_tile + row * 2;
-                    if (leader && has_res && part < nchunks && o_base + part * 32 < epi.O) {
-                        load_res(o_base + part * 32);
-                        if (MODE == kModeGeneral && part + parts < nchunks && o_base + (part + parts) * 32 < epi.O)
-                            tma_prefetch_l2_2d(&map_r, o_base + (part + parts) * 32, c1);
-                    }
                     bool stg_ok = true;
 #pragma unroll 1
-                    for (int c = part; c < nchunks; c += parts) {
+                    for (int c = part; c < nchunks; c += parts, ++stg_count) {
                         const int col0 = c * 32;
                         const bool real = o_base + col0 < epi.O;      // false: nothing but the int8 output's channel padding
+                        const int t = stg_count & (kp.stg_tiles - 1);
+                        const uint32_t r_row = base + kp.stg_off + (uint32_t)(quad * kp.stg_tiles + t) * kStageF32Bytes + (uint32_t)row * 128u + (uint32_t)(row & 7) * 16u;
+                        const uint32_t tile_phase = (uint32_t)(kp.stg_tiles == 2 ? stg_count >> 1 : stg_count) & 1u;
                         int v[32];
+                        if (real) tmem_ld32(taddr0 + (uint32_t)(DUAL && !concat ? BN + col0 : col0), v);
+                        // the tile is free, and holds the residual if there is one
+                        stg_ok = __all_sync(0xffffffffu, mbar_wait(bar_stg + 8 * (quad * 2 + t), tile_phase, abort_flag));
+                        if (!stg_ok) { tmem_ld_wait(); break; }
                         if constexpr (DUAL) {
                             // the projection's 32 channels of this pixel, dequantized (+ bias), into the thread's own row of
                             // the fp32 tile -- where a tensor-map load would have put a residual
                             if (real && !concat) {
-                                tmem_ld32(taddr0 + (uint32_t)(BN + col0), v);
                                 tmem_ld_wait();
-                                const bool bias2 = dual.bias2 != nullptr;
 #pragma unroll
                                 for (int j4 = 0; j4 < 8; ++j4) {
                                     const float4 d4 = *reinterpret_cast<const float4 *>(t_dq + 2 * BN + col0 + 4 * j4);
                                     const float4 b4 = *reinterpret_cast<const float4 *>(t_dq + 3 * BN + col0 + 4 * j4);
                                     float4 f;
-                                    f.x = __fmul_rn(__int2float_rn(v[4 * j4 + 0]), d4.x);
-                                    f.y = __fmul_rn(__int2float_rn(v[4 * j4 + 1]), d4.y);
-                                    f.z = __fmul_rn(__int2float_rn(v[4 * j4 + 2]), d4.z);
-                                    f.w = __fmul_rn(__int2float_rn(v[4 * j4 + 3]), d4.w);
-                                    if (bias2) { f.x = __fadd_rn(f.x, b4.x); f.y = __fadd_rn(f.y, b4.y); f.z = __fadd_rn(f.z, b4.z); f.w = __fadd_rn(f.w, b4.w); }
-                                    r_row[j4 ^ key] = f;
+                                    f.x = __fadd_rn(__fmul_rn(__int2float_rn(v[4 * j4 + 0]), d4.x), b4.x);
+                                    f.y = __fadd_rn(__fmul_rn(__int2float_rn(v[4 * j4 + 1]), d4.y), b4.y);
+                                    f.z = __fadd_rn(__fmul_rn(__int2float_rn(v[4 * j4 + 2]), d4.z), b4.z);
+                                    f.w = __fadd_rn(__fmul_rn(__int2float_rn(v[4 * j4 + 3]), d4.w), b4.w);
+                                    sts128(r_row ^ (uint32_t)(j4 * 16), f);
+                                }
+                                tmem_ld32(taddr0 + (uint32_t)col0, v);
+                            }
+                        }
+                        uint32_t q[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+                        bool fine = true;
+                        if (real) {
+                            tmem_ld_wait();
+                            with_act_flag(act, epi.even, [&](auto a, auto even) {
+                                fine = staged_chunk_t<TSB_VAL(a), TSB_VAL(even), EPI == kEpiStagedAfter>(v, t_dq + col0, t_bias + col0, epi.leaky, r_row, has_res || (DUAL && !concat), has_i8, rs, q);
+                            });
+                        }
+                        if (has_i8) {
+                            // the previous chunk's int8 tile has been read
+                            stg_ok = __all_sync(0xffffffffu, mbar_wait(bar_stg + 8 * (4 * kQuads + quad), (uint32_t)(stg_count + 1) & 1u, abort_flag));
+                            if (!stg_ok) break;
+                            sts128(q_row, q[0], q[1], q[2], q[3]);
+                            sts128(q_row + 16, q[4], q[5], q[6], q[7]);
+                            const uint32_t nchw0 = (uint32_t)(img * epi.O + o_base + col0) * (uint32_t)epi.P + (uint32_t)p;
+                            if (real && live && (!fine || (epi.tail && nchw0 + 31u * (uint32_t)epi.P >= epi.rne_limit))) {
+                                // NaN or a value beyond the int32 range (they quantize to -128 in the reference), or an
+                                // element of the tensor's tail, which rounds the other way: exactly, from the fp32 results
+                                for (int j = 0; j < 32 && o_base + col0 + j < epi.O; ++j) {
+                                    float f;
+                                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"((r_row ^ (uint32_t)((j >> 2) * 16)) + (uint32_t)(j & 3) * 4u) : "memory");
+                                    const int b = q8(f, rs, epi.even && nchw0 + (uint32_t)j * (uint32_t)epi.P < epi.rne_limit);
+                                    asm volatile("st.shared.u8 [%0], %1;" ::"r"(q_row + (uint32_t)j), "r"(b) : "memory");
                                 }
                             }
                         }
-                        if (real) tmem_ld32(taddr0 + (uint32_t)col0, v);
-                        else {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = 0;
-                        }
-                        if (real && has_res) {
-                            if (!mbar_wait(rbar, stg_phase[0], abort_flag)) { stg_ok = false; }
-                            stg_phase[0] ^= 1u;
-                        }
-                        if (real) tmem_ld_wait();
-                        bool fine = true;
-                        if (stg_ok) {
-                            with_act_flags(act, epi.even, epi.res_after, [&](auto a, auto even, auto after) {
-                                fine = staged_chunk_t<TSB_VAL(a), TSB_VAL(even), TSB_VAL(after)>(v, t_dq + col0, t_bias + col0, epi.leaky, r_row, key, real && (has_res || (DUAL && !concat)), has_f32, q_row, has_i8, rs);
-                            });
-                            // the tensor's last count % 8 elements round the other way (fix_tail): the chunk goes element by element
-                            if (epi.tail && real && live && ((uint32_t)(img * epi.O + min(o_base + col0 + 31, epi.O - 1)) * (uint32_t)epi.P + (uint32_t)p) >= epi.rne_limit) fine = false;
-                        }
                         fence_async_smem();
-                        // all four warps have written their rows; the OR says whether any value needs the exact slow path
-                        const bool redo = bar_or(bar_id, 128, !fine || !stg_ok);
-                        if (leader) {
-                            if (!redo) {
-                                if (has_f32 && real) store_tile(&map_of, stg, o_base + col0);
-                                if (has_i8) store_tile(&map_oi, q_addr, o_base + col0);
-                                bulk_commit();
-                            }
-                            bulk_wait_read();                                        // the tiles may be overwritten
-                            const int cn = c + parts;
-                            if (has_res && cn < nchunks && o_base + cn * 32 < epi.O) load_res(o_base + cn * 32);
-                            // and the residual box after that one on its way into L2
-                            const int cp = cn + parts;
-                            if (has_res && MODE == kModeGeneral && cp < nchunks && o_base + cp * 32 < epi.O) tma_prefetch_l2_2d(&map_r, o_base + cp * 32, c1);
-                        }
-                        if (redo) {
-                            // NaN or a value beyond the int32 range (they quantize to -128 in the reference), or a load that
-                            // did not arrive: this chunk goes element by element, straight to global memory
-                            for (int j = 0; j < 32; ++j) {
-                                const int o = o_base + col0 + j;
-                                const int a = real ? tmem_ld1(taddr0 + (uint32_t)(col0 + j)) : 0;
-                                int a2 = 0;
-                                if constexpr (DUAL) a2 = (real && !concat) ? tmem_ld1(taddr0 + (uint32_t)(BN + col0 + j)) : 0;
-                                if (!live) continue;
-                                if (DUAL && !concat && o < epi.O) {
-                                    float r = __fmul_rn(__int2float_rn(a2), t_dq[2 * BN + col0 + j]);
-                                    if constexpr (DUAL) { if (dual.bias2) r = __fadd_rn(r, t_dq[3 * BN + col0 + j]); }
-                                    epilogue_store_value(epi, img, o, p, a, r, true);
-                                } else if (o < epi.O) epilogue_store_one(epi, img, o, p, a);
-                                else if (has_i8 && epi.i8_nhwc && o < epi.out_cp) epi.out_i8[(size_t)m * epi.out_cp + o] = 0;
-                            }
-                        }
-                        // the next chunk's writes must not overtake the leader's wait above; with a residual the load it
-                        // issues afterwards orders them, otherwise a second barrier does
-                        if (!(has_res && c + parts < nchunks && o_base + (c + parts) * 32 < epi.O)) asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_stg + 8 * (2 * kQuads + quad * 2 + t));     // this warp's rows are written
                     }
-                    if (!stg_ok && !*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 7); }
+                    if (!stg_ok) {
+                        if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 7); }
+                        break;
+                    }
                 } else {
 #pragma unroll 1
                 for (int c = part; c < BN / CW; c += parts) {
@@ -1674,7 +1726,7 @@ int launch(const Config &cfg, const CUtensorMap &ma, const CUtensorMap &mb, cons
         TSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynamicSmem));
         configured.fetch_or(bit, std::memory_order_release);
     }
-    TSB_CUDA(launch_pdl(kernel, dim3(cfg.grid), dim3(kThreads), cfg.dyn_smem, stream, ma, mb, mr, mof, moi, kp, epi, dual));
+    TSB_CUDA(launch_pdl(kernel, dim3(cfg.grid), dim3(cta_threads(EPI)), cfg.dyn_smem, stream, ma, mb, mr, mof, moi, kp, epi, dual));
     TSB_LAUNCHED("conv_i8_tc_kernel");
     return TSB_OK;
 }
@@ -1683,13 +1735,15 @@ int launch(const Config &cfg, const CUtensorMap &ma, const CUtensorMap &mb, cons
 // X(BN, BK, SWAP, MODE, EPI, DUAL)
 #define TSB_TC_NORMAL(X, BN_, BK_, MODE_)                                                                                    \
     X(BN_, BK_, false, MODE_, kEpiGeneric, false) X(BN_, BK_, false, MODE_, kEpiF32Nchw, false)                             \
-    X(BN_, BK_, false, MODE_, kEpiI8Nhwc, false) X(BN_, BK_, false, MODE_, kEpiStaged, false)
+    X(BN_, BK_, false, MODE_, kEpiI8Nhwc, false) X(BN_, BK_, false, MODE_, kEpiStaged, false)                                 \
+    X(BN_, BK_, false, MODE_, kEpiStagedAfter, false)
 #define TSB_TC_SWAPPED(X, BN_, BK_)                                                                                          \
     X(BN_, BK_, true, kModeGeneral, kEpiGeneric, false) X(BN_, BK_, true, kModeGeneral, kEpiF32Nchw, false)                 \
     X(BN_, BK_, true, kModeGeneral, kEpiI8Nhwc, false) X(BN_, BK_, true, kModeGeneral, kEpiNhwc, false)                     \
     X(BN_, BK_, true, kModePatch, kEpiGeneric, false) X(BN_, BK_, true, kModePatch, kEpiF32Nchw, false)                     \
     X(BN_, BK_, true, kModePatch, kEpiI8Nhwc, false)
-#define TSB_TC_PAIR(X, BN_, BK_) X(BN_, BK_, false, kModeGeneral, kEpiStaged, true) X(BN_, BK_, false, kModeGeneral, kEpiI8Nhwc, true)
+#define TSB_TC_PAIR(X, BN_, BK_)                                                                                             \
+    X(BN_, BK_, false, kModeGeneral, kEpiStaged, true) X(BN_, BK_, false, kModeGeneral, kEpiStagedAfter, true) X(BN_, BK_, false, kModeGeneral, kEpiI8Nhwc, true)
 #define TSB_TC_PART_0(X) TSB_TC_NORMAL(X, 64, 64, kModeGeneral) TSB_TC_NORMAL(X, 64, 128, kModeGeneral) TSB_TC_NORMAL(X, 64, 64, kModePatch)
 #define TSB_TC_PART_1(X) TSB_TC_NORMAL(X, 128, 64, kModeGeneral) TSB_TC_NORMAL(X, 128, 128, kModeGeneral) TSB_TC_NORMAL(X, 64, 128, kModePatch)
 #define TSB_TC_PART_2(X) TSB_TC_NORMAL(X, 256, 64, kModeGeneral) TSB_TC_NORMAL(X, 256, 128, kModeGeneral)
