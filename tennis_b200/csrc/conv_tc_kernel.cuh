@@ -912,12 +912,15 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        // Like the issuers below, the whole warp walks the tiles and one elected lane issues: 64 images of ResNet-50 1.155 -> 1.137 ms, 8 images
+        // 0.424 -> 0.404; CSPDarknet53, 16 images 2.58 -> 2.46 ms, one image 0.570 -> 0.534.
+        {
             int stage = 0, stage_lo = 0, stage_alt = ring;                  // absolute stage, first stage of its ring; the other ring's
             uint32_t phase = 0, phase_alt = 0;
             auto next_stage = [&]() { if (++stage == stage_lo + ring) { stage = stage_lo; phase ^= 1u; } };
             bool ok = true;
             int cur_n = -1, w_loads = 0;
+            const uint32_t tx_bytes = (uint32_t)kp.kgroup * (kp.b_resident ? kPixBytes : kPixBytes + kWgtBytes);
             for (int i = 0; i < my_tiles && ok; ++i) {
                 if (i > 0 && issuers > 1) {                                 // the next tile is the other issuer's
                     const int s = stage; stage = stage_alt; stage_alt = s;
@@ -933,16 +936,18 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 const int wc = ow * kp.sw - kp.pad_l, hc = oh * kp.sh - kp.pad_t;
                 if (kp.b_resident && n_tile != cur_n) {
                     // (re)load the whole weight tile; wait until the MMAs that read the previous one are done
-                    if (w_loads > 0 && !mbar_wait(bar_bfree, (uint32_t)(w_loads - 1) & 1u, abort_flag)) {
+                    if (w_loads > 0 && !mbar_wait_warp(bar_bfree, (uint32_t)(w_loads - 1) & 1u, abort_flag)) {
                         if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 5); }
                         break;
                     }
-                    mbar_arrive_expect_tx(bar_bfull, (uint32_t)(k_iters + k_sc) * kWgtBytes);
-                    if constexpr (DUAL)
-                        for (int it = 0; it < k_sc; ++it)
-                            tma_load_2d(w_res + (uint32_t)it * kWgtBytes, &dual.map_b2, bar_bfull, it * BK, n_tile * CH);
-                    for (int it = 0; it < k_iters; ++it)
-                        tma_load_2d(w_res + (uint32_t)(k_sc + it) * kWgtBytes, &map_b, bar_bfull, it * BK, n_tile * CH);
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(bar_bfull, (uint32_t)(k_iters + k_sc) * kWgtBytes);
+                        if constexpr (DUAL)
+                            for (int it = 0; it < k_sc; ++it)
+                                tma_load_2d(w_res + (uint32_t)it * kWgtBytes, &dual.map_b2, bar_bfull, it * BK, n_tile * CH);
+                        for (int it = 0; it < k_iters; ++it)
+                            tma_load_2d(w_res + (uint32_t)(k_sc + it) * kWgtBytes, &map_b, bar_bfull, it * BK, n_tile * CH);
+                    }
                     cur_n = n_tile;
                     ++w_loads;
                 }
@@ -951,13 +956,15 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     const int p_r = kp.d_tiles_w.div(p_rem), p_c = p_rem - p_r * kp.patch_tiles_w;
                     const int h0 = p_r * (PIX / 8) - kp.pad_t, w0 = p_c * 8 - kp.pad_l;
                     for (int cb = 0; cb < kp.Cp && ok; cb += BK) {
-                        if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
+                        if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
                             if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 1); }
                             ok = false;
                             break;
                         }
-                        mbar_arrive_expect_tx(bar_full + 8 * stage, kp.patch_bytes);
-                        tma_load_4d(base + stage * kp.stage_bytes, &map_a, bar_full + 8 * stage, cb, w0, h0, p_img);
+                        if (elect_one()) {
+                            mbar_arrive_expect_tx(bar_full + 8 * stage, kp.patch_bytes);
+                            tma_load_4d(base + stage * kp.stage_bytes, &map_a, bar_full + 8 * stage, cb, w0, h0, p_img);
+                        }
                         next_stage();
                     }
                 } else if (MODE == kModeRows) {
@@ -969,17 +976,19 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         const int r_img = kp.d_OH.div(row_id), r_oh = row_id - r_img * kp.rows_OH;
                         int kh_lo, kh_hi;
                         rows_span(kp, r_oh, kh_lo, kh_hi);
-                        if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
+                        if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
                             if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 1); }
                             break;
                         }
                         const int ih_lo = r_oh * kp.sh - kp.pad_t + kh_lo * kp.dh;
                         const uint32_t bytes = (uint32_t)((kh_hi - kh_lo) * kp.dh) * (uint32_t)kp.rows_stride_h +
                                                (uint32_t)(kp.rows_segs - 1 - seg) * (PIX * 16) + kp.rows_bytes;
-                        mbar_arrive_expect_tx(bar_full + 8 * stage, bytes);
-                        bulk_load(base + stage * kp.stage_bytes,
-                                  kp.rows_x + r_img * kp.rows_stride_n + ih_lo * kp.rows_stride_h + (long long)seg * (PIX * 16),
-                                  bytes, bar_full + 8 * stage);
+                        if (elect_one()) {
+                            mbar_arrive_expect_tx(bar_full + 8 * stage, bytes);
+                            bulk_load(base + stage * kp.stage_bytes,
+                                      kp.rows_x + r_img * kp.rows_stride_n + ih_lo * kp.rows_stride_h + (long long)seg * (PIX * 16),
+                                      bytes, bar_full + 8 * stage);
+                        }
                         next_stage();
                     }
                 } else {
@@ -988,17 +997,19 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         const int wc2 = ow * dual.sw2, hc2 = oh * dual.sh2;   // the projection: 1x1, no padding
                         for (int cb = 0; cb < dual.Cp2; cb += BK) {
                             if (gk == 0) {
-                                if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
+                                if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
                                     if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 1); }
                                     ok = false;
                                     break;
                                 }
-                                mbar_arrive_expect_tx(bar_full + 8 * stage, (uint32_t)kp.kgroup * (kp.b_resident ? kPixBytes : kPixBytes + kWgtBytes));
                             }
                             const uint32_t sp = base + stage * kp.stage_bytes + (uint32_t)gk * kp.unit_bytes, sw = sp + kPixBytes;
-                            if (dual.a2_tiled) tma_load_2d(sp, &dual.map_a2, bar_full + 8 * stage, cb, m0);
-                            else tma_load_im2col_4d(sp, &dual.map_a2, bar_full + 8 * stage, cb, wc2, hc2, img, (uint16_t)0, (uint16_t)0);
-                            if (!kp.b_resident) tma_load_2d(sw, &dual.map_b2, bar_full + 8 * stage, cb, n_tile * CH);
+                            if (elect_one()) {
+                                if (gk == 0) mbar_arrive_expect_tx(bar_full + 8 * stage, tx_bytes);
+                                if (dual.a2_tiled) tma_load_2d(sp, &dual.map_a2, bar_full + 8 * stage, cb, m0);
+                                else tma_load_im2col_4d(sp, &dual.map_a2, bar_full + 8 * stage, cb, wc2, hc2, img, (uint16_t)0, (uint16_t)0);
+                                if (!kp.b_resident) tma_load_2d(sw, &dual.map_b2, bar_full + 8 * stage, cb, n_tile * CH);
+                            }
                             if (++gk == kp.kgroup) {
                                 gk = 0;
                                 next_stage();
@@ -1009,21 +1020,23 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         for (int kw = 0; kw < kp.KW && ok; ++kw)
                             for (int cb = 0; cb < kp.Cp; cb += BK) {
                                 if (gk == 0) {
-                                    if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
+                                    if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
                                         if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 1); }
                                         ok = false;
                                         break;
                                     }
-                                    mbar_arrive_expect_tx(bar_full + 8 * stage, (uint32_t)kp.kgroup * (kp.b_resident ? kPixBytes : kPixBytes + kWgtBytes));
                                 }
                                 const uint32_t sp = base + stage * kp.stage_bytes + (uint32_t)gk * kp.unit_bytes, sw = sp + kPixBytes;
-                                if (kp.a_tiled)
-                                    tma_load_2d(sp, &map_a, bar_full + 8 * stage, cb, m0);
-                                else
-                                    tma_load_im2col_4d(sp, &map_a, bar_full + 8 * stage, cb, wc, hc, img,
-                                                       (uint16_t)(kw * kp.dw), (uint16_t)(kh * kp.dh));
-                                if (!kp.b_resident)
-                                    tma_load_2d(sw, &map_b, bar_full + 8 * stage, (kh * kp.KW + kw) * kp.Cp + cb, n_tile * CH);
+                                if (elect_one()) {
+                                    if (gk == 0) mbar_arrive_expect_tx(bar_full + 8 * stage, tx_bytes);
+                                    if (kp.a_tiled)
+                                        tma_load_2d(sp, &map_a, bar_full + 8 * stage, cb, m0);
+                                    else
+                                        tma_load_im2col_4d(sp, &map_a, bar_full + 8 * stage, cb, wc, hc, img,
+                                                           (uint16_t)(kw * kp.dw), (uint16_t)(kh * kp.dh));
+                                    if (!kp.b_resident)
+                                        tma_load_2d(sw, &map_b, bar_full + 8 * stage, (kh * kp.KW + kw) * kp.Cp + cb, n_tile * CH);
+                                }
                                 if (++gk == kp.kgroup) {
                                     gk = 0;
                                     next_stage();
