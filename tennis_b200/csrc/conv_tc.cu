@@ -140,13 +140,16 @@ bool wants_staging(const View &v, const EpiParams &epi) {
 // Shared memory of the staged epilogue: per quad `tiles` fp32 tiles and an int8 tile.
 static uint32_t staged_bytes(int tiles) { return tiles ? kQuads * ((uint32_t)tiles * kStageF32Bytes + kStageI8Bytes) : 0u; }
 
+// bytes of K from which on a layer of few tiles is split
+constexpr int kSplitMinK = 2048;
+
 // tiles: fp32 tiles per quad of the staged epilogue, 0: not staged
 static Config plan_config(const View &v, const Tuning &tune, int sm_count, int orientation, int tiles_per_quad) {
     const ConvGeom &g = v.g;
     Config c;
     c.bk = (g.Cp % 128 == 0) ? 128 : 64;
     const int64_t M = (int64_t)g.N * g.OH * g.OW;
-    const uint32_t stg_bytes = staged_bytes(tiles_per_quad), budget = kSmemBudget - stg_bytes;
+    uint32_t stg_bytes = staged_bytes(tiles_per_quad), budget = kSmemBudget - stg_bytes;
     // An MMA instruction costs the same 128 cycles for any N up to 256, so N should be 256 whenever possible.
     // Normal orientation: 128 pixels on M, up to 256 output channels on N.  Swapped orientation: channels on M,
     // 256 (or 128) pixels on N -- it halves the MMA count of narrow layers but its epilogue (one channel per thread)
@@ -164,7 +167,14 @@ static Config plan_config(const View &v, const Tuning &tune, int sm_count, int o
         return (eff >= 0.7 || tune.patch == 2) && w_all + 2 * patch_bytes <= budget;
     };
     const int bn_normal = g.O > 128 ? 256 : (g.O > 64 ? 128 : 64);
-    if (v.rows) c.swap = 0;
+    // Split-K where clusters of kSplit CTAs, one per 128 x 128 tile, fit the GPU at once and a tile has K enough to pay for the exchange of
+    // the partial sums (some 3 us with the cluster's launch).  Measured alone, cold, split against whole: 3x3 512 -> 512 at 7 x 7, 8 images,
+    // 11.5 / 16 us; 3x3 512 -> 512 at 19 x 19, one image, 15 / 19 us; 3x3 256 -> 256 at 38 x 38 13.4 / 14.5; 1x1 1024 -> 256 at 14 x 14,
+    // 8 images, 10 / 8.  Patch mode, which loads an activation once and not once per tap, stays ahead where it fits (256 -> 256 at 14 x 14,
+    // 8 images, 9.5 / 10.5).  CSPDarknet53 of one image 0.535 -> 0.519 ms, ResNet-50 of 8 images 0.398 -> 0.395.
+    const bool split = orientation < 0 && tune.orientation != 2 && tune.patch != 2 && !v.fold && g.KH * g.KW * g.Cp >= kSplitMinK &&
+                       ceil_div64(M, kBM) * ceil_div(g.O, 128) * kSplit <= sm_count - sm_count / 8;
+    if (v.rows || split) c.swap = 0;
     else if (orientation >= 0) c.swap = orientation;
     else if (tune.orientation) c.swap = tune.orientation == 2 && g.O <= 128;
     // narrow multi-tap layers: swapped fills the MMA's N, but where patch mode applies the normal orientation with its
@@ -195,9 +205,13 @@ static Config plan_config(const View &v, const Tuning &tune, int sm_count, int o
         c.pix = kBM;
         c.ch = c.bn;
     }
+    if (split && !patch_fits(c.pix, c.ch)) {
+        c.split = 1;
+        c.bn = c.ch = 128;
+    }
     c.num_m_tiles = v.rows ? g.N * g.OH * v.rows_segs : (int)ceil_div64(M, c.pix);
     c.num_n_tiles = ceil_div(g.O, c.ch);
-    if (patch_fits(c.pix, c.ch)) {
+    if (!c.split && patch_fits(c.pix, c.ch)) {
         const int th = c.pix / 8;
         c.patch = 1;
         c.patch_tiles_w = ceil_div(g.OW, 8); c.patch_tiles_h = ceil_div(g.OH, th);
@@ -205,7 +219,8 @@ static Config plan_config(const View &v, const Tuning &tune, int sm_count, int o
         c.num_m_tiles = g.N * c.patch_tiles_w * c.patch_tiles_h;
     }
     const int64_t tiles = (int64_t)c.num_m_tiles * c.num_n_tiles;
-    c.grid = (int)(tiles < sm_count ? tiles : sm_count);
+    c.grid = c.split ? (int)tiles * kSplit : (int)(tiles < sm_count ? tiles : sm_count);
+    if (c.split) budget = kSmemBudget - (stg_bytes = staged_bytes(1));   // the partial sums of the other CTAs arrive in the quads' fp32 tiles
     // shared-memory plan: keep the CTA's whole weight tile resident when it is small enough to leave room for
     // at least four activation stages; otherwise stream activations and weights together
     // raw-row mode stages, per output row, the KH staged image rows under all its segments of 128 sliding windows
@@ -215,14 +230,14 @@ static Config plan_config(const View &v, const Tuning &tune, int sm_count, int o
     const uint32_t w_bytes = (uint32_t)c.ch * c.bk;
     const uint32_t k_iters = (uint32_t)g.KH * g.KW * (g.Cp / c.bk);
     const uint32_t w_total = k_iters * w_bytes;
-    const bool want_resident = v.rows || c.patch || tiles > c.grid;  // pays off only when a CTA runs several tiles
+    const bool want_resident = v.rows || c.patch || (tiles > c.grid && !c.split);  // pays off only when a CTA runs several tiles
     // (raw-row mode always keeps its weights resident; make_view admitted it only where two row stages fit beside them)
     const uint32_t min_stages = v.rows ? 2 : 4;
     // K blocks per stage (im2col / tiled loads only): the MMA issuer pays a barrier wait and a commit per stage, which
     // costs it more than the MMAs of one K block take when N is small, so short K blocks are grouped -- as long as the
     // group divides the K blocks of a tile, stays within 48 KB and leaves at least three stages.
     auto group_for = [&](uint32_t unit, uint32_t room) {
-        if (c.patch || v.rows) return 1;
+        if (c.patch || v.rows || c.split) return 1;
         for (int gsz = 4; gsz >= 2; gsz /= 2)
             if (k_iters % (uint32_t)gsz == 0 && (uint32_t)gsz * unit <= 48 * 1024 && room / ((uint32_t)gsz * unit) >= 3) return gsz;
         return 1;
@@ -245,11 +260,12 @@ static Config plan_config(const View &v, const Tuning &tune, int sm_count, int o
         c.bar_off = (uint32_t)c.stages * c.stage_bytes;
     }
     // the staged epilogue's tiles (1024-byte aligned for the 128B swizzle) sit between the pipeline and the barriers
-    c.staging = c.swap ? 0 : tiles_per_quad;
+    c.staging = c.swap ? 0 : (c.split ? std::min(tiles_per_quad, 1) : tiles_per_quad);
     // The more of a group's quads work on one tile, the closer together the CTA's copies lie in memory; but a quad needs a
     // chunk of its own (32 channels), and the tiles of a deep K come too slowly for one group to wait for each in turn.
     c.stg_groups = v.a_tiled ? (c.bn >= 128 ? 1 : 2) : (c.bn >= 128 ? 2 : 4);
-    if (c.staging) {
+    if (c.split) c.stg_groups = 1;
+    if (c.staging || c.split) {
         c.stg_off = (c.bar_off + 1023u) & ~1023u;
         c.bar_off = c.stg_off + stg_bytes;
     }
@@ -546,7 +562,7 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
     // take the staged class, below
     if (!epi.out_acc && (epi.out_f32 || epi.residual) && epi.f32_nhwc && i8_fast && (const void *)epi.residual != (const void *)epi.out_f32 && cfg.swap && !cfg.patch)
         epi_mode = kEpiNhwc;
-    const int mode = cfg.patch ? kModePatch : (v.rows ? kModeRows : kModeGeneral);
+    const int mode = cfg.patch ? kModePatch : (v.rows ? kModeRows : (cfg.split ? kModeSplit : kModeGeneral));
     // Pixel-major fp32 residual (the shortcut of a residual block, as large as the output): a tensor map over it lets the
     // epilogue prefetch the boxes it is about to read into L2.  The map is not used for loads, so a failure to encode one
     // only switches the prefetch off.

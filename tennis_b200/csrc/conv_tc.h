@@ -43,6 +43,7 @@ struct Config {
     int pix = 0, ch = 0;              // pixels and output channels per tile
     int num_m_tiles = 0, num_n_tiles = 0;
     int patch = 0;                    // this configuration runs in patch mode
+    int split = 0;                    // the K blocks of a tile are shared out over a cluster of CTAs
     int patch_tiles_w = 0, patch_tiles_h = 0, patch_pw = 0, patch_ph = 0;   // tiles per image, patch extent in pixels
     int grid = 0;                     // persistent CTAs
     // shared-memory plan of the kernel

@@ -1,4 +1,4 @@
-// One group of instances of the tensor-core kernel: compiled once per group with -DTSB_TC_PART=0..9.
+// One group of instances of the tensor-core kernel: compiled once per group with -DTSB_TC_PART=0..10.
 #include "conv_tc_kernel.cuh"
 
 namespace tsb {

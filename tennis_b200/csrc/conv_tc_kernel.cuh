@@ -89,6 +89,40 @@ __device__ __forceinline__ bool elect_one() {
     return on != 0;
 }
 
+// ---- clusters (split-K): CTAs that write to each other's shared memory
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// the address of `addr` (this CTA's shared memory) in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+    uint32_t out;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
+    return out;
+}
+__device__ __forceinline__ void sts128_cluster(uint32_t addr, int a, int b, int c, int d) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// an arrival on another CTA's barrier that publishes what the cluster can see of this thread's writes
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// mbar_wait that sees what the other CTAs of the cluster wrote before they arrived
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    const long long t0 = clock64();
+    for (uint32_t spin = 0;; ++spin) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+        if ((spin & 255u) == 255u) {
+            if (*abort_flag) return false;
+            if (clock64() - t0 > 4000000000LL) return false;
+        }
+    }
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -187,6 +221,17 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int (&v)[32]) {
           "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr) : "memory");
 }
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const int (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
+        ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+          "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+          "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(taddr) : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor of a K-major tile whose rows are one swizzle span (BK bytes) wide:
@@ -272,6 +317,7 @@ __host__ __device__ constexpr bool is_staged(int epi) { return epi == kEpiStaged
 __host__ __device__ constexpr int cta_threads(int epi) { return 32 * (kCopyWarp0 + (is_staged(epi) ? 4 : 0)); }
 constexpr uint32_t kStageF32Bytes = kBM * 32 * 4;   // one staged fp32 tile: 128 pixels x 32 channels, 128-byte rows, swizzle 128B
 constexpr uint32_t kStageI8Bytes = kBM * 32;        // one staged int8 tile: 128 pixels x 32 channels, 32-byte rows
+constexpr int kSplit = 4;                           // CTAs that share the K blocks of a tile in split-K mode
 constexpr int kQuads = 4;                           // the sixteen epilogue warps form four quads of one warp per lane quarter
 
 // (a layer without a bias adds a zero: the same value up to the sign of a zero, which the operators' results are compared up
@@ -760,7 +806,10 @@ __device__ __forceinline__ void rows_span(const KernelParams &kp, int oh, int &k
     kh_hi = min(kp.KH - 1, kp.d_dh.div(kp.rows_H - 1 - top));
 }
 
-constexpr int kModeGeneral = 0, kModeRows = 1, kModePatch = 2;
+// kModeSplit: as kModeGeneral, but the K blocks of a tile are shared out over the kSplit CTAs of a cluster, for layers whose tiles
+// leave most of the GPU idle: one SM takes in its operands at about 60 bytes a cycle however many there are.  BN = 128 only: each of the
+// four CTAs adds up and finishes one 32-channel chunk of the tile (int32 sums are exact in any order).
+constexpr int kModeGeneral = 0, kModeRows = 1, kModePatch = 2, kModeSplit = 3;
 
 // Projected-shortcut kernels (DUAL): a second, 1x1 convolution over the same output pixels (the projection shortcut of a
 // residual block: its own input, weights, dequantize scales and bias) runs in the same tile, into a second accumulator,
@@ -780,8 +829,8 @@ constexpr int kMaxStages = 24;
 constexpr uint32_t kMaxDynamicSmem = 227 * 1024;
 
 // barriers, in this order: full[stages], empty[stages], tmem_full[4], tmem_empty[4], b_full, b_free, and for the staged
-// epilogue's tiles ready[4 quads][2], full[4][2], int8_free[4]
-__host__ __device__ constexpr uint32_t num_barriers(int stages) { return 2u * (uint32_t)stages + 2u * kMaxAccBufs + 2u + 5u * kQuads; }
+// epilogue's tiles ready[4 quads][2], full[4][2], int8_free[4]; split-K: the partial sums of the other CTAs are here
+__host__ __device__ constexpr uint32_t num_barriers(int stages) { return 2u * (uint32_t)stages + 2u * kMaxAccBufs + 2u + 5u * kQuads + 1u; }
 
 // PIX pixels x CH channels per tile.  Normal orientation: the pixel tile is the MMA's A operand (M = 128 pixels), the
 // weight tile its B operand (N = BN channels).  Swapped orientation: the weight tile is A (M = 128 channels, rows
@@ -797,6 +846,8 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                   const __grid_constant__ CUtensorMap map_oi, const __grid_constant__ KernelParams kp,
                   const __grid_constant__ EpiParams epi,
                   const __grid_constant__ std::conditional_t<DUAL, DualParams, NoDual> dual) {
+    constexpr bool SPLIT = MODE == kModeSplit;
+    static_assert(!SPLIT || (!SWAP && BN == 32 * kSplit), "split-K: one 32-channel chunk of the tile per CTA of the cluster");
     static_assert(!DUAL || (!SWAP && MODE == kModeGeneral), "projected-shortcut kernels: normal orientation, general mode");
     static_assert(SWAP ? !is_staged(EPI) : EPI != kEpiNhwc, "pixel-major fp32 tensors: staged tiles where a thread owns a pixel");
     constexpr int PIX = SWAP ? BN : kBM;      // pixels per tile
@@ -817,6 +868,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const uint32_t bar_bfull = bar_tempty + 8 * kMaxAccBufs;
     const uint32_t bar_bfree = bar_bfull + 8;
     const uint32_t bar_stg = bar_bfree + 8;     // the staged epilogue's
+    const uint32_t bar_parts = bar_stg + 8 * 5 * kQuads;    // split-K
     const uint32_t slot_off = kp.bar_off + 8 * num_barriers(kStages);
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(base_ptr + slot_off);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(base_ptr + slot_off + 4);
@@ -834,9 +886,11 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     // This CTA's tiles.  Streaming weights: tiles blockIdx.x, +gridDim.x, ... with the channel tile running fastest.
     // Resident weights: one contiguous range of the channel-major tile order, so the weight tile changes at most a
     // few times.
+    const int rank = SPLIT ? (int)blockIdx.x % kSplit : 0;                     // split-K: the CTA of its cluster (clusters are consecutive CTAs)
+    const int k_lo = SPLIT ? k_iters * rank / kSplit : 0, k_hi = SPLIT ? k_iters * (rank + 1) / kSplit : k_iters;
     const int tile_lo = kp.b_resident ? (int)((long long)blockIdx.x * total_tiles / gridDim.x) : 0;
     const int tile_hi = kp.b_resident ? (int)((long long)(blockIdx.x + 1) * total_tiles / gridDim.x) : 0;
-    const int my_tiles = kp.b_resident ? tile_hi - tile_lo : (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int my_tiles = SPLIT ? 1 : kp.b_resident ? tile_hi - tile_lo : (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
     // Accumulator buffers in use = epilogue groups: as many as tensor memory holds (kBufs), but no more than this CTA has
     // tiles -- a CTA with a single tile puts all sixteen epilogue warps on it.
     // (a projected-shortcut tile holds two accumulators: buffers 2a and 2a+1 of logical buffer a)
@@ -848,7 +902,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const int t = tile_lo + i;
             n_tile = kp.d_m_tiles.div(t); m_tile = t - n_tile * kp.num_m_tiles;
         } else {
-            const int t = (int)blockIdx.x + i * (int)gridDim.x;
+            const int t = SPLIT ? (int)blockIdx.x / kSplit : (int)blockIdx.x + i * (int)gridDim.x;
             m_tile = kp.d_n_tiles.div(t); n_tile = t - m_tile * kp.num_n_tiles;
         }
     };
@@ -862,7 +916,8 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const bool tempty = t >= kMaxAccBufs && t < 2 * kMaxAccBufs;
             const int stg = t - (2 * kMaxAccBufs + 2);                                // staged tiles: ready, full, int8 free
             const bool full = stg >= 2 * kQuads && stg < 4 * kQuads;
-            mbar_init(bar_full + 8 * i, tempty ? kEpiThreads / groups : (full ? 4 : 1));
+            const bool parts_in = stg == 5 * kQuads;                                  // four warps of each of the other CTAs
+            mbar_init(bar_full + 8 * i, tempty ? kEpiThreads / groups : (full ? 4 : (parts_in ? 4 * (kSplit - 1) : 1)));
         }
         if (lane == 0) {
             *abort_flag = 0;
@@ -906,6 +961,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int ring = issuers > 1 ? kStages / kIssuers : kStages;
     tc_fence_before();
     __syncthreads();
+    if constexpr (SPLIT) cluster_arrive();      // this CTA's barriers are initialised
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_sync();   // everything above touched only shared and tensor memory
@@ -1016,9 +1072,15 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                             }
                         }
                     }
-                    for (int kh = 0; kh < kp.KH && ok; ++kh)
-                        for (int kw = 0; kw < kp.KW && ok; ++kw)
-                            for (int cb = 0; cb < kp.Cp; cb += BK) {
+                    int kh_0 = 0, kw_0 = 0, cb_0 = 0, left = k_hi - k_lo;       // (split-K: from the middle of a tap to the middle of another)
+                    if constexpr (SPLIT) {
+                        const int blocks = kp.Cp / BK, tap = k_lo / blocks;
+                        kh_0 = tap / kp.KW; kw_0 = tap - kh_0 * kp.KW; cb_0 = (k_lo - tap * blocks) * BK;
+                    }
+                    for (int kh = kh_0; kh < kp.KH && ok; ++kh, kw_0 = 0)
+                        for (int kw = kw_0; kw < kp.KW && ok; ++kw, cb_0 = 0)
+                            for (int cb = cb_0; cb < kp.Cp; cb += BK) {
+                                if (SPLIT && left-- == 0) { ok = false; break; }
                                 if (gk == 0) {
                                     if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
                                         if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 1); }
@@ -1259,7 +1321,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                             }
                         }
                     };
-                    for (int it = 0; it < k_iters + k_sc; it += G) {
+                    for (int it = k_lo; it < k_hi + k_sc; it += G) {
                         if (DUAL && it == k_sc && !concat) { d_tmem -= BN; accumulate = 0u; }   // the main convolution's accumulator
                         TSB_CYC_START;
                         if (!mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag)) {
@@ -1269,7 +1331,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         }
                         TSB_CYC_ADD(cyc_full);
                         tc_fence_after();
-                        if (it == 0 && me == 0) TSB_TRACE(local, 3);
+                        if (it == k_lo && me == 0) TSB_TRACE(local, 3);
                         TSB_CYC_START;
                         if (elect_one()) {
                             if (G == 4) issue_stage(std::integral_constant<int, 4>());
@@ -1325,6 +1387,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 const int ch_end = min(w.o_base + BN, max(epi.O, has_i8 ? epi.out_cp : 0));
                 w.nchunks = ch_end > w.o_base ? (ch_end - w.o_base + 31) >> 5 : 0;
                 w.c = part;
+                if (SPLIT && part != rank) w.nchunks = 0;                       // another CTA of the cluster finishes this chunk
                 w.c1 = m_tile * PIX; w.c2 = 0; w.c3 = 0;                          // general: [pixel][channel]
                 if (MODE == kModeRows) {                                        // [image row][ow][channel]
                     const int row_id = kp.d_segs.div(m_tile);
@@ -1411,6 +1474,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             decode(local, m_tile, n_tile);
             const int o_base = n_tile * CH;
             const int slot = DUAL ? 2 * acc : acc;          // first accumulator buffer of this tile
+            if constexpr (SPLIT) cluster_wait();    // ... and those of the other CTAs, to which partial sums will go
             float *t_dq = table + (DUAL ? 2 * group : group) * 2 * BN, *t_bias = t_dq + BN;
             if (!SWAP && n_tile != table_n) {
                 // this group's table of per-channel scales and biases: rebuilt only when the channel tile changes (never, for
@@ -1442,6 +1506,38 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             if (kp.trace && kp.trace[255] != 0) { tc_fence_before(); mbar_arrive(bar_tempty + 8 * acc); continue; }
 #endif
             const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(slot * BN);
+            if constexpr (SPLIT) {
+                // The sixteen warps hold one tile: part = chunk = the CTA that finishes it.  A warp whose chunk another CTA finishes sends
+                // its 32 x 32 partial sums there, into the slot of this CTA (16-byte pieces of consecutive rows side by side), and
+                // is done; the warps of this CTA's chunk add the three slots to their own accumulators, in tensor memory, and go on.
+                // (Slot i lies in the fp32 tile of quad i, which the staged epilogue does not use here unless i is this CTA.)
+                int v[32];
+                tmem_ld32(taddr0 + (uint32_t)(part * 32), v);
+                tmem_ld_wait();
+                const uint32_t slots = base + kp.stg_off + (uint32_t)row * 16u;
+                if (part != rank) {
+                    const uint32_t to = map_to_rank(slots + (uint32_t)rank * kStageF32Bytes, (uint32_t)part);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) sts128_cluster(to + (uint32_t)j * (kBM * 16), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(map_to_rank(bar_parts, (uint32_t)part));
+                    continue;
+                }
+                if (!__all_sync(0xffffffffu, mbar_wait_cluster(bar_parts, 0u, abort_flag))) {
+                    if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 9); }
+                    break;
+                }
+                for (int q = 0; q < kSplit; ++q) {
+                    if (q == rank) continue;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int4 a = *reinterpret_cast<const int4 *>(base_ptr + kp.stg_off + (uint32_t)q * kStageF32Bytes + (uint32_t)(j * kBM + row) * 16u);
+                        v[4 * j] += a.x; v[4 * j + 1] += a.y; v[4 * j + 2] += a.z; v[4 * j + 3] += a.w;
+                    }
+                }
+                tmem_st32(taddr0 + (uint32_t)(part * 32), v);
+            }
             if constexpr (!SWAP) {
                 int m = m_tile * PIX + row;
                 bool live = m < kp.M_total;
@@ -1735,6 +1831,12 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
     tc_fence_before();
     __syncthreads();
+    if constexpr (SPLIT) {
+        // Nobody may write to, or arrive in, a CTA that has left.  One that has its partial sums gets no more of either; one that gave up
+        // stays until the others have left or given up (threads that have exited count as arrived).
+        if (warp < kEpiWarp0 || warp >= kCopyWarp0) cluster_wait();     // (the epilogue warps have done so above)
+        if (*abort_flag) { cluster_arrive(); cluster_wait(); }
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
@@ -1757,7 +1859,8 @@ int launch(const Config &cfg, const CUtensorMap &ma, const CUtensorMap &mb, cons
         TSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynamicSmem));
         configured.fetch_or(bit, std::memory_order_release);
     }
-    TSB_CUDA(launch_pdl(kernel, dim3(cfg.grid), dim3(cta_threads(EPI)), cfg.dyn_smem, stream, ma, mb, mr, mof, moi, kp, epi, dual));
+    TSB_CUDA(launch_pdl_cluster(MODE == kModeSplit ? kSplit : 1, kernel, dim3(cfg.grid), dim3(cta_threads(EPI)), cfg.dyn_smem, stream, ma, mb, mr, mof, moi,
+                                kp, epi, dual));
     TSB_LAUNCHED("conv_i8_tc_kernel");
     return TSB_OK;
 }
@@ -1786,9 +1889,10 @@ int launch(const Config &cfg, const CUtensorMap &ma, const CUtensorMap &mb, cons
 #define TSB_TC_PART_8(X) TSB_TC_SWAPPED(X, 256, 64) TSB_TC_SWAPPED(X, 256, 128)
 #define TSB_TC_PART_9(X)                                                                                                     \
     TSB_TC_PAIR(X, 64, 64) TSB_TC_PAIR(X, 64, 128) TSB_TC_PAIR(X, 128, 64) TSB_TC_PAIR(X, 128, 128) TSB_TC_PAIR(X, 256, 64) TSB_TC_PAIR(X, 256, 128)
+#define TSB_TC_PART_10(X) TSB_TC_NORMAL(X, 128, 64, kModeSplit) TSB_TC_NORMAL(X, 128, 128, kModeSplit)
 #define TSB_TC_ALL(X)                                                                                                        \
     TSB_TC_PART_0(X) TSB_TC_PART_1(X) TSB_TC_PART_2(X) TSB_TC_PART_3(X) TSB_TC_PART_4(X) TSB_TC_PART_5(X) TSB_TC_PART_6(X)  \
-    TSB_TC_PART_7(X) TSB_TC_PART_8(X) TSB_TC_PART_9(X)
+    TSB_TC_PART_7(X) TSB_TC_PART_8(X) TSB_TC_PART_9(X) TSB_TC_PART_10(X)
 
 }  // namespace tc
 }  // namespace tsb
