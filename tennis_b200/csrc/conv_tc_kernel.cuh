@@ -907,17 +907,20 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
     };
 
+    // raw rows of several tiles: both issuers consume one ring (below)
+    const bool shared_ring = MODE == kModeRows && kp.rows_segs > 1;
     if (threadIdx.x == 0) TSB_TRACE(0, 7);
     if (warp == 0) {
         // one barrier per lane and step (a single thread takes 0.3 us for the eighty of them); the descriptors' first fetch
         // overlaps the wait for the previous kernel
         for (int i = lane; i < (int)num_barriers(kStages); i += 32) {
-            const int t = i - 2 * kStages;                                            // full, empty: one arrival each
+            const int t = i - 2 * kStages;                                            // full, empty: one arrival each (empty: one per issuer of a shared ring)
             const bool tempty = t >= kMaxAccBufs && t < 2 * kMaxAccBufs;
             const int stg = t - (2 * kMaxAccBufs + 2);                                // staged tiles: ready, full, int8 free
             const bool full = stg >= 2 * kQuads && stg < 4 * kQuads;
             const bool parts_in = stg == 5 * kQuads;                                  // four warps of each of the other CTAs
-            mbar_init(bar_full + 8 * i, tempty ? kEpiThreads / groups : (full ? 4 : (parts_in ? 4 * (kSplit - 1) : 1)));
+            const bool empty = i >= kStages && t < 0;
+            mbar_init(bar_full + 8 * i, empty ? (shared_ring ? kIssuers : 1) : tempty ? kEpiThreads / groups : (full ? 4 : (parts_in ? 4 * (kSplit - 1) : 1)));
         }
         if (lane == 0) {
             *abort_flag = 0;
@@ -938,27 +941,28 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             tap16[t] = (uint32_t)((kh * kp.dh * kp.patch_pw + kw * kp.dw) * BK) >> 4;
         }
     }
-    // How many warps issue MMAs, each for every such tile of the CTA.  One where tiles share state that one thread has to order -- a
-    // raw-row stage shared by the segments of an output row, or resident weights that are replaced inside this CTA's tile
-    // range -- and where the ring of stages has no room for a tile of each issuer.
+    // How many warps issue MMAs, each for every such tile of the CTA.  One where tiles share state that one thread has to order --
+    // resident weights that are replaced inside this CTA's tile range -- and where the ring of stages has no room for a tile of each issuer.
     // Each issuer has a ring of stages of its own (stages [i * kStages / issuers, ...) for issuer i), which the producer fills for
     // that issuer's tiles.  A barrier wait names a phase by its parity only; in a ring that nobody else consumes, an issuer
     // has itself seen the round before the one it waits for.  (With one ring for both, an issuer could arrive at a stage while the
     // other issuer's tile of the round before was still being loaded -- loads complete out of order -- and pass its wait.)
+    // (Raw-row stages that several tiles of an output row share are the exception: there both issuers walk all rows through one ring,
+    // and a stage is free when both have said so -- each sees every fill.)
     int issuers = 1;
     if (my_tiles > 1 && warp <= kIssuers) {
         const int spt = MODE == kModePatch ? kp.Cp / BK : (MODE == kModeRows ? 1 : (k_iters + k_sc) / kp.kgroup);   // stages a tile consumes
-        bool shared_state = MODE == kModeRows && kp.rows_segs > 1;
+        bool shared_state = false;
         if (kp.b_resident && kp.num_n_tiles > 1) {
             int first_m, first_n, last_m, last_n;
             decode(0, first_m, first_n);
             decode(my_tiles - 1, last_m, last_n);
-            shared_state = shared_state || first_n != last_n;
+            shared_state = first_n != last_n;
         }
         // (an issuer must also own its accumulator buffers: with a single logical buffer one thread takes every tile)
-        if (!shared_state && kStages >= kIssuers * spt && !(DUAL && nbuf < kIssuers)) issuers = kIssuers;
+        if (!shared_state && (shared_ring || kStages >= kIssuers * spt) && !(DUAL && nbuf < kIssuers)) issuers = kIssuers;
     }
-    const int ring = issuers > 1 ? kStages / kIssuers : kStages;
+    const int ring = issuers > 1 && !shared_ring ? kStages / kIssuers : kStages;
     tc_fence_before();
     __syncthreads();
     if constexpr (SPLIT) cluster_arrive();      // this CTA's barriers are initialised
@@ -978,7 +982,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             int cur_n = -1, w_loads = 0;
             const uint32_t tx_bytes = (uint32_t)kp.kgroup * (kp.b_resident ? kPixBytes : kPixBytes + kWgtBytes);
             for (int i = 0; i < my_tiles && ok; ++i) {
-                if (i > 0 && issuers > 1) {                                 // the next tile is the other issuer's
+                if (i > 0 && issuers > 1 && !shared_ring) {                              // the next tile is the other issuer's
                     const int s = stage; stage = stage_alt; stage_alt = s;
                     const uint32_t p = phase; phase = phase_alt; phase_alt = p;
                     stage_lo = ring - stage_lo;
@@ -1128,9 +1132,36 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const uint32_t base16 = base >> 4, stage16 = kp.stage_bytes >> 4, wres16 = w_res >> 4, unit16 = kp.unit_bytes >> 4;
             const int resident = kp.b_resident;
             bool ok = true;
-            int rows_seg_first = 0;
-            const int me = warp - 1, stage_lo = me * ring;
+            const int me = warp - 1, stage_lo = shared_ring ? 0 : me * ring;
             int stage = stage_lo; uint32_t phase = 0;
+            // raw rows: the output row whose stage comes next, the segment its copy starts at, whether it is there; the last row of this CTA
+            int rows_next = 0, rows_seg_first = 0, rows_last = 0;
+            bool rows_held = false;
+            if (shared_ring) {
+                int m_tile, n_tile;
+                decode(0, m_tile, n_tile);
+                rows_next = kp.d_segs.div(m_tile); rows_seg_first = m_tile - rows_next * kp.rows_segs;
+                decode(my_tiles - 1, m_tile, n_tile);
+                rows_last = kp.d_segs.div(m_tile);
+            }
+            auto rows_pass = [&]() {            // on to the next row; this one's stage is free when the MMAs have read it
+                if (elect_one()) {
+                    tc_commit(bar_empty + 8 * stage);
+                    if (shared_ring && issuers == 1) tc_commit(bar_empty + 8 * stage);      // for the issuer that is not there
+                }
+                if (++stage == stage_lo + ring) { stage = stage_lo; phase ^= 1u; }
+                ++rows_next;
+                rows_held = false;
+                rows_seg_first = 0;
+            };
+            auto rows_wait = [&]() {
+                if (!rows_held && !mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag)) {
+                    if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 3); }
+                    return false;
+                }
+                rows_held = true;
+                return true;
+            };
             int w_loads = resident ? 1 : 0;   // without shared state the resident weights are loaded exactly once
             int cur_n = -1;
             // patch mode with up to nine filter taps (3x3, 1x3 ...): the taps' window offsets live in registers
@@ -1238,23 +1269,24 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     const int row_id = kp.d_segs.div(m_tile), seg = m_tile - row_id * kp.rows_segs;
                     int kh_lo, kh_hi;
                     rows_span(kp, row_id - kp.d_OH.div(row_id) * kp.rows_OH, kh_lo, kh_hi);
-                    if (seg == 0 || local == me) {     // the stage of this output row: loaded once, used by all its segments
-                        TSB_CYC_START;
-                        if (!mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag)) {
-                            if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 3); }
-                            break;
+                    if (shared_ring) {
+                        // a row without a tile of this issuer (the CTA's first, with a single tile, of the other's) is passed by
+                        while (issuers > 1 && ok && rows_next < row_id) {
+                            ok = rows_wait();
+                            if (ok) rows_pass();
                         }
-                        TSB_CYC_ADD(cyc_full);
-                        tc_fence_after();
-                        rows_seg_first = seg;
+                        st16 = base16 + (uint32_t)stage * stage16;
                     }
+                    ok = ok && rows_wait();
+                    if (!ok) break;
+                    tc_fence_after();
                     if (me == 0) TSB_TRACE(local, 3);
                     // sliding descriptor (no swizzle, LBO 16, SBO 128): only its address field changes from row to row
                     const uint64_t dslide = smem_desc_sliding(0);
                     const uint32_t row16 = (uint32_t)kp.dh * (uint32_t)(kp.rows_stride_h >> 4);
                     // filter row kh reads the staged row (kh - kh_lo); rows outside [kh_lo, kh_hi] meet no input row
                     const uint32_t a16_0 = st16 + (uint32_t)(seg - rows_seg_first) * PIX - (uint32_t)kh_lo * row16;
-                    const bool row_done = seg == kp.rows_segs - 1 || local == my_tiles - 1;
+                    const bool row_done = seg + issuers >= kp.rows_segs || local + issuers >= my_tiles;    // this issuer's last tile of the row
                     if (elect_one()) {
                     if (kp.KH <= 8) {
                         // straight-line code for the filter heights in use (a predicated-off MMA still costs the issuing
@@ -1299,9 +1331,8 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                             }
                         }
                     }
-                    if (row_done) tc_commit(bar_empty + 8 * stage);
                     }
-                    if (row_done && ++stage == stage_lo + ring) { stage = stage_lo; phase ^= 1u; }
+                    if (row_done) rows_pass();
                 } else {
                     // general mode: a stage holds kgroup K blocks; one wait, kgroup * BK/32 MMAs in a row, one commit
                     uint32_t w16 = wres16;
@@ -1355,6 +1386,11 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     if (nn != cur_n && elect_one()) tc_commit(bar_bfree);  // the resident weights may be replaced
                 }
                 if (me == 0) TSB_TRACE(local, 4);
+            }
+            // ... and so is the last one
+            while (shared_ring && issuers > 1 && ok && rows_next <= rows_last) {
+                ok = rows_wait();
+                if (ok) rows_pass();
             }
             if (me == 0) TSB_CYC_REPORT((my_tiles + issuers - 1) / issuers);
         }
