@@ -99,8 +99,12 @@ bool make_view(const ConvGeom &g, const Tuning &tune, View *view, const char **w
     }
     v.a_tiled = (!v.fold && g.KH == 1 && g.KW == 1 && g.sh == 1 && g.sw == 1 && g.pad_t == 0 && g.pad_l == 0 &&
                  g.OH == g.H && g.OW == g.W) ? 1 : 0;
-    v.patch = (!v.fold && !v.a_tiled && g.sh == 1 && g.sw == 1 && g.KH * g.KW > 1 && (g.KW - 1) * g.dw + 8 <= 256 &&
-               (g.KH - 1) * g.dh + 32 <= 256 && tune.patch != 1) ? 1 : 0;
+    if (!v.fold && !v.a_tiled && g.KH * g.KW > 1 && tune.patch != 1) {
+        if (g.sh == 1 && g.sw == 1 && (g.KW - 1) * g.dw + 8 <= 256 && (g.KH - 1) * g.dh + 32 <= 256) v.patch = 1;
+        // (stride 2 over 64 padded channels: 297 rows of 128 bytes a tile instead of the 1152 im2col rows of 64 bytes, at some 4.5 cycles a row;
+        // CSPDarknet53, whose 32 -> 64 and 64 -> 128 layers at 608 and 304 take it, 16 images 2.37 -> 2.21 ms, one image 0.511 -> 0.501)
+        else if (g.sh == 2 && g.sw == 2 && g.dh == 1 && g.dw == 1 && g.Cp == 64 && g.W % 2 == 0 && g.KW <= 128 && g.KH <= 128) v.patch = 2;
+    }
     const ConvGeom &t = v.g;
     v.weight_bytes = (size_t)t.O * t.KH * t.KW * t.Cp;
     // im2col tensor maps take box corners in [-128,127], filter offsets in [0,255] and traversal strides up to 8
@@ -156,13 +160,28 @@ static Config plan_config(const View &v, const Tuning &tune, int sm_count, int o
     // is dearer, so it is taken where it measured faster: multi-tap filters with at most 64 output channels.
     // patch mode under a given tile shape: most of each 8 x (pix/8) tile inside the image, and the whole weight tile
     // in shared memory beside at least two patches (tune.patch == 2 drops the first condition)
+    // (extent of a patch in pixels or pixel pairs; a row of it in bytes)
+    auto patch_extent = [&](int pix, int *pw, int *ph) {
+        const int th = pix / 8;
+        if (v.patch == 2) {
+            *pw = 8 + (g.KW - 1 - g.pad_l >= 0 ? (g.KW - 1 - g.pad_l) / 2 : -((g.pad_l - g.KW + 2) / 2)) + (g.pad_l + 1) / 2;
+            *ph = (th - 1) * 2 + g.KH;
+        } else {
+            *pw = 8 + (g.KW - 1) * g.dw;
+            *ph = th + (g.KH - 1) * g.dh;
+        }
+    };
+    const int patch_row = v.patch == 2 ? 128 : c.bk;
     auto patch_fits = [&](int pix, int ch) {
         if (!v.patch) return false;
+        // (the swapped kernel has no fast path for pixel-major fp32 tensors in patch mode, which is what the swapped plan is kept for)
+        if (v.patch == 2 && c.swap && tune.patch != 2) return false;
         const int th = pix / 8;
         const int tiles_w = ceil_div(g.OW, 8), tiles_h = ceil_div(g.OH, th);
-        const int pw = 8 + (g.KW - 1) * g.dw, ph = th + (g.KH - 1) * g.dh;
+        int pw, ph;
+        patch_extent(pix, &pw, &ph);
         const double eff = (double)(g.OH * g.OW) / ((double)tiles_w * tiles_h * pix);
-        const uint64_t patch_bytes = (uint64_t)round_up(pw * ph * c.bk, 1024);
+        const uint64_t patch_bytes = (uint64_t)round_up(pw * ph * patch_row, 1024);
         const uint64_t w_all = (uint64_t)g.KH * g.KW * g.Cp * (uint64_t)ch;
         return (eff >= 0.7 || tune.patch == 2) && w_all + 2 * patch_bytes <= budget;
     };
@@ -213,9 +232,9 @@ static Config plan_config(const View &v, const Tuning &tune, int sm_count, int o
     c.num_n_tiles = ceil_div(g.O, c.ch);
     if (!c.split && patch_fits(c.pix, c.ch)) {
         const int th = c.pix / 8;
-        c.patch = 1;
+        c.patch = v.patch;
         c.patch_tiles_w = ceil_div(g.OW, 8); c.patch_tiles_h = ceil_div(g.OH, th);
-        c.patch_pw = 8 + (g.KW - 1) * g.dw; c.patch_ph = th + (g.KH - 1) * g.dh;
+        patch_extent(c.pix, &c.patch_pw, &c.patch_ph);
         c.num_m_tiles = g.N * c.patch_tiles_w * c.patch_tiles_h;
     }
     const int64_t tiles = (int64_t)c.num_m_tiles * c.num_n_tiles;
@@ -225,7 +244,7 @@ static Config plan_config(const View &v, const Tuning &tune, int sm_count, int o
     // at least four activation stages; otherwise stream activations and weights together
     // raw-row mode stages, per output row, the KH staged image rows under all its segments of 128 sliding windows
     // (127 pixel strides of 16 bytes plus one window in the last segment)
-    const uint32_t p_bytes = c.patch ? (uint32_t)round_up(c.patch_pw * c.patch_ph * c.bk, 1024) : v.rows ? (uint32_t)round_up((g.KH - 1) * g.dh * (int)v.stride_h + (v.rows_segs - 1) * kBM * 16 + (kBM - 1) * 16 + c.bk, 128)
+    const uint32_t p_bytes = c.patch ? (uint32_t)round_up(c.patch_pw * c.patch_ph * patch_row, 1024) : v.rows ? (uint32_t)round_up((g.KH - 1) * g.dh * (int)v.stride_h + (v.rows_segs - 1) * kBM * 16 + (kBM - 1) * 16 + c.bk, 128)
                                     : (uint32_t)c.pix * c.bk;
     const uint32_t w_bytes = (uint32_t)c.ch * c.bk;
     const uint32_t k_iters = (uint32_t)g.KH * g.KW * (g.Cp / c.bk);
@@ -381,12 +400,13 @@ int encode_activation_map(const View &v, const Config &cfg, const int8_t *x, CUt
     if (reinterpret_cast<uintptr_t>(x) % 16) return fail(TSB_ERR_INVALID_ARGUMENT, "staged activations must be 16-byte aligned");
     const ConvGeom &g = v.g;
     if (cfg.patch) {
-        cuuint64_t dims4[4] = {(cuuint64_t)g.Cp, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)g.N};
-        cuuint64_t strides4[3] = {v.stride_w, v.stride_h, v.stride_n};
-        cuuint32_t box4[4] = {(cuuint32_t)cfg.bk, (cuuint32_t)cfg.patch_pw, (cuuint32_t)cfg.patch_ph, 1};
+        const cuuint64_t pair = cfg.patch == 2 ? 2 : 1;      // pixels per row of the patch
+        cuuint64_t dims4[4] = {(cuuint64_t)g.Cp * pair, (cuuint64_t)g.W / pair, (cuuint64_t)g.H, (cuuint64_t)g.N};
+        cuuint64_t strides4[3] = {v.stride_w * pair, v.stride_h, v.stride_n};
+        cuuint32_t box4[4] = {(cuuint32_t)(cfg.bk * pair), (cuuint32_t)cfg.patch_pw, (cuuint32_t)cfg.patch_ph, 1};
         cuuint32_t estr4[4] = {1, 1, 1, 1};
         CUresult r4 = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<int8_t *>(x), dims4, strides4, box4,
-                                     estr4, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(cfg.bk),
+                                     estr4, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for((int)(cfg.bk * pair)),
                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r4 != CUDA_SUCCESS) return fail(TSB_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled(activation patches) failed with %d", (int)r4);
         return TSB_OK;
@@ -538,7 +558,8 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
     kp.rows_x = nullptr;
     kp.patch = cfg.patch; kp.OH = g.OH;
     kp.patch_tiles_w = std::max(1, cfg.patch_tiles_w); kp.patch_tiles_hw = std::max(1, cfg.patch_tiles_w * cfg.patch_tiles_h);
-    kp.patch_pw = cfg.patch_pw; kp.patch_bytes = (uint32_t)(cfg.patch_pw * cfg.patch_ph * cfg.bk);
+    kp.patch_pw = cfg.patch_pw; kp.patch_bytes = (uint32_t)(cfg.patch_pw * cfg.patch_ph * (cfg.patch == 2 ? 128 : cfg.bk));
+    kp.patch_left = cfg.patch == 2 ? (g.pad_l + 1) / 2 : g.pad_l;
     kp.d_tiles_w = FastDiv((uint32_t)kp.patch_tiles_w); kp.d_tiles_hw = FastDiv((uint32_t)kp.patch_tiles_hw);
     if (cfg.patch && !cfg.b_resident) return fail(TSB_ERR_UNSUPPORTED, "patch mode needs resident weights");
     if (v.rows) {

@@ -22,12 +22,15 @@ namespace tc {
 //            8 pixels wide and pix/8 pixels high; one tiled tensor-map load per channel block brings the input patch under
 //            it (halo included, zero-filled outside the image) and every filter tap reads its shifted window out of that
 //            patch, so an activation byte is loaded once per tile instead of once per tap.  Needs resident weights.
+//  patch == 2 (stride 2, 64 padded channels, even width): the same over pixel PAIRS, i.e. over the tensor [N][H][W/2][128].  The
+//            even and the odd pixels that the taps of a strided filter alternate between are the halves of 128-byte rows, and the
+//            windows of neighbouring output pixels are neighbouring rows again.
 struct View {
     ConvGeom g;          // geometry handed to the kernel and the tensor maps
     ConvGeom real;       // geometry of the operator
     int fold = 0;
     int rows = 0;        // raw-row mode
-    int patch = 0;       // patch mode is possible for this geometry
+    int patch = 0;       // patch mode is possible for this geometry: 1 pixels, 2 pixel pairs
     int rows_segs = 0;   // tiles per output row in raw-row mode
     int a_tiled = 0;     // 1x1 / stride 1 / no padding: the activations are the [M][Cp] matrix itself, loaded as 2-D tiles
     int cpix = 0;        // bytes per pixel of the folded staging
@@ -42,7 +45,7 @@ struct Config {
     int swap = 0;                     // 1: channels on the MMA's M side and pixels on its N side
     int pix = 0, ch = 0;              // pixels and output channels per tile
     int num_m_tiles = 0, num_n_tiles = 0;
-    int patch = 0;                    // this configuration runs in patch mode
+    int patch = 0;                    // this configuration runs in patch mode (View::patch)
     int split = 0;                    // the K blocks of a tile are shared out over a cluster of CTAs
     int patch_tiles_w = 0, patch_tiles_h = 0, patch_pw = 0, patch_ph = 0;   // tiles per image, patch extent in pixels
     int grid = 0;                     // persistent CTAs

@@ -750,12 +750,13 @@ struct KernelParams {
     uint32_t rows_bytes;   // bytes copied per tile and filter row
     long long rows_stride_h, rows_stride_n;   // bytes between staged rows / images
     const int8_t *rows_x;  // the folded staging
-    // patch mode (patch != 0; stride-1 filters with several taps): a tile is 8 pixels wide and PIX/8 pixels high; ONE
+    // patch mode (patch != 0; filters with several taps, of stride 1 or, patch == 2, stride 2 and 64 padded channels): a tile is 8 pixels wide and PIX/8 pixels high; ONE
     // tiled tensor-map load per channel block brings the input patch under it, halo included, and every filter tap reads
     // its shifted window out of that patch through a descriptor whose start is moved by whole pixels
     int patch;
     int patch_tiles_w, patch_tiles_hw;        // tiles across an image, tiles per image
-    int patch_pw;                             // patch width in pixels: 8 + (KW-1)*dw
+    int patch_pw;                             // patch width in pixels (8 + (KW-1)*dw) or pixel pairs
+    int patch_left;                           // columns (pairs) of the patch left of the tile's first pixel (of its pair): pad_l or (pad_l+1)/2
     uint32_t patch_bytes;                     // bytes of one patch (one channel block)
     int OH;
     FastDiv d_tiles_w, d_tiles_hw;
@@ -804,6 +805,17 @@ __device__ __forceinline__ void rows_span(const KernelParams &kp, int oh, int &k
     const int top = oh * kp.sh - kp.pad_t;                 // input row under filter row 0
     kh_lo = top >= 0 ? 0 : kp.d_dh.div(-top + kp.dh - 1);
     kh_hi = min(kp.KH - 1, kp.d_dh.div(kp.rows_H - 1 - top));
+}
+
+// Patch mode: distance of filter tap (kh, kw)'s window from the start of a patch, in bytes.  In a patch of pixel pairs (stride 2) a row of
+// shared memory is an even and an odd pixel of 64 channels each, so a tap takes one half of the pair it falls on.
+template <int BK>
+__device__ __forceinline__ uint32_t patch_tap(const KernelParams &kp, int kh, int kw) {
+    if (kp.patch == 2) {
+        const int col = kw - kp.pad_l;
+        return (uint32_t)((kh * kp.patch_pw + (col >> 1) + kp.patch_left) * 128 + (col & 1) * 64);
+    }
+    return (uint32_t)((kh * kp.dh * kp.patch_pw + kw * kp.dw) * BK);
 }
 
 // kModeSplit: as kModeGeneral, but the K blocks of a tile are shared out over the kSplit CTAs of a cluster, for layers whose tiles
@@ -938,7 +950,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     if (MODE == kModePatch && threadIdx.x >= 32 * kEpiWarp0) {
         for (int t = (int)threadIdx.x - 32 * kEpiWarp0; t < kp.KH * kp.KW; t += kEpiThreads) {
             const int kh = t / kp.KW, kw = t - kh * kp.KW;
-            tap16[t] = (uint32_t)((kh * kp.dh * kp.patch_pw + kw * kp.dw) * BK) >> 4;
+            tap16[t] = patch_tap<BK>(kp, kh, kw) >> 4;
         }
     }
     // How many warps issue MMAs, each for every such tile of the CTA.  One where tiles share state that one thread has to order --
@@ -1014,7 +1026,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 if (MODE == kModePatch) {
                     const int p_img = kp.d_tiles_hw.div(m_tile), p_rem = m_tile - p_img * kp.patch_tiles_hw;
                     const int p_r = kp.d_tiles_w.div(p_rem), p_c = p_rem - p_r * kp.patch_tiles_w;
-                    const int h0 = p_r * (PIX / 8) - kp.pad_t, w0 = p_c * 8 - kp.pad_l;
+                    const int h0 = p_r * (PIX / 8) * kp.sh - kp.pad_t, w0 = p_c * 8 - kp.patch_left;
                     for (int cb = 0; cb < kp.Cp && ok; cb += BK) {
                         if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
                             if (!*abort_flag) { *abort_flag = 1; atomicExch(kp.status, 1); }
@@ -1171,7 +1183,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 int kh = 0, kw = 0;
 #pragma unroll
                 for (int t = 0; t < 9; ++t) {
-                    tapreg[t] = (MODE == kModePatch && t < taps) ? (uint32_t)((kh * kp.dh * kp.patch_pw + kw * kp.dw) * BK) >> 4 : 0u;
+                    tapreg[t] = (MODE == kModePatch && t < taps) ? patch_tap<BK>(kp, kh, kw) >> 4 : 0u;
                     if (++kw == kp.KW) { kw = 0; ++kh; }
                 }
             }
@@ -1203,7 +1215,8 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 uint32_t accumulate = 0;
                 if (MODE == kModePatch) {
                     const int n_cb = kp.Cp / BK;
-                    const uint64_t dhi_patch = smem_desc_hi<BK>((uint32_t)kp.patch_pw * BK);   // next tile row = next patch row
+                    // next tile row = next patch row, or the next but one of pixel pairs
+                    const uint64_t dhi_patch = kp.patch == 2 ? smem_desc_hi<128>(2u * (uint32_t)kp.patch_pw * 128u) : smem_desc_hi<BK>((uint32_t)kp.patch_pw * BK);
                     const uint32_t hi_patch = (uint32_t)(dhi_patch >> 32), hi_plain = (uint32_t)(dhi >> 32);
                     const uint32_t wtap16 = (uint32_t)n_cb * kWgt16;                          // next tap of the resident weights
                     for (int cbi = 0; cbi < n_cb && ok; ++cbi) {
