@@ -315,10 +315,14 @@ class Conv2DQuantized(Operator):
         self.field("dialations", OPTIONAL)
         self.field("dequantize_scales", REQUIRED)
         self._kernel = kernel
+        # plans by what they were made from, this operator's own configuration included: attributes that are set again do not
+        # meet a plan of the ones before them, and a plan that a captured graph refers to stays where it is
         self._plans = {}
-        self._dq_dev = None
+        self._dq_dev = {}
+        self._config = None
 
     def init(self):
+        self._config = object()           # no plan is of a configuration that fails a check below
         super().init()
         fmt = self.get("format")
         padding = np.asarray(self.get("padding")).astype(np.int32)
@@ -351,6 +355,7 @@ class Conv2DQuantized(Operator):
             raise EjectionException("%s do not support dialations: %s" % (self.op, _to_string(dilation)))
         self.padding4x2, self.stride4, self.dilation4 = p, stride, dilation
         self.dequantize_scales = np.asarray(self.get("dequantize_scales"), dtype=np.float32).reshape(-1)
+        self._config = (fmt, p.tobytes(), stride.tobytes(), dilation.tobytes(), self.padding_value, self.dequantize_scales.tobytes())
 
     def _geometry(self):
         p, s, d = self.padding4x2, self.stride4, self.dilation4
@@ -382,8 +387,8 @@ class Conv2DQuantized(Operator):
         plan = None
         if len(inputs) == 2:
             x, w = inputs
-            # a plan was made for these shapes and types only after they had passed every check
-            key = (x.shape, w.shape, w.data_ptr(), x.dtype, w.dtype, x.device)
+            # a plan was made for this configuration, these shapes and types only after they had passed every check
+            key = (self._config, x.shape, w.shape, w.data_ptr(), x.dtype, w.dtype, x.device)
             plan = self._plans.get(key)
         if plan is None:
             self.infer(inputs)
@@ -396,11 +401,12 @@ class Conv2DQuantized(Operator):
                 raise EjectionException(e.message)
             plan.set_weights(w, stream)
             self._plans[key] = plan
-        if self._dq_dev is None or self._dq_dev.device != x.device:
-            self._dq_dev = torch.from_numpy(self.dequantize_scales).to(x.device)
+        dq = self._dq_dev.get((self._config, x.device))
+        if dq is None:
+            dq = self._dq_dev[self._config, x.device] = torch.from_numpy(self.dequantize_scales.copy()).to(x.device)
         x = x.contiguous()
         out = torch.empty(plan.out_shape, dtype=torch.float32, device=x.device)
-        plan.run(x, LAYOUT_NCHW, self._dq_dev, out_f32=out, out_acc=out_acc, stream=stream)
+        plan.run(x, LAYOUT_NCHW, dq, out_f32=out, out_acc=out_acc, stream=stream)
         return out
 
 
