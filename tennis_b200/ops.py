@@ -300,6 +300,11 @@ def _to_string(arr):
     return "[" + ", ".join(str(int(v)) for v in arr) + "]"
 
 
+def _writes(t):
+    """How often a tensor's memory was written so far; None where PyTorch does not count (inference tensors)."""
+    return None if t.is_inference() else t._version
+
+
 class Conv2DQuantized(Operator):
     """Operator "conv2d_quantized" on the GPU: int8 NCHW x int8 OIHW -> fp32 NCHW."""
 
@@ -384,13 +389,15 @@ class Conv2DQuantized(Operator):
         return [("float32", (x.shape[0], OH, OW, w.shape[0]))]
 
     def run(self, inputs, stream=None, out_acc=None):
-        plan = None
+        """The weights are packed when they are new and when they were written since, as far as PyTorch counts writes (a write
+        through ``.data`` or a raw pointer is not counted)."""
+        kept = None
         if len(inputs) == 2:
             x, w = inputs
             # a plan was made for this configuration, these shapes and types only after they had passed every check
-            key = (self._config, x.shape, w.shape, w.data_ptr(), x.dtype, w.dtype, x.device)
-            plan = self._plans.get(key)
-        if plan is None:
+            key = (self._config, x.shape, w.shape, w.stride(), w.data_ptr(), x.dtype, w.dtype, x.device)
+            kept = self._plans.get(key)
+        if kept is None:
             self.infer(inputs)
             if self.format != "NCHW":
                 raise EjectionException("Conv2D_quantized only support NCHW")  # conv2d_quantized_core.cpp:131-133
@@ -400,7 +407,14 @@ class Conv2DQuantized(Operator):
             except TsbError as e:
                 raise EjectionException(e.message)
             plan.set_weights(w, stream)
-            self._plans[key] = plan
+            # (the tensor is kept, so that its address stays its own)
+            self._plans[key] = [plan, w, _writes(w)]
+        else:
+            plan = kept[0]
+            writes = _writes(w)
+            if writes is None or writes != kept[2]:
+                plan.set_weights(w, stream)
+                kept[2] = writes
         dq = self._dq_dev.get((self._config, x.device))
         if dq is None:
             dq = self._dq_dev[self._config, x.device] = torch.from_numpy(self.dequantize_scales.copy()).to(x.device)

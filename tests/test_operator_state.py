@@ -83,3 +83,55 @@ def test_attributes_set_again_are_checked_again(monkeypatch):
     op.set("padding", np.zeros((3, 2), dtype=np.int32))
     with pytest.raises(ops.EjectionException):
         op.init()
+
+
+def test_weights_written_between_calls_are_used(monkeypatch):
+    x, w, dq = tensors()
+    op = operator(monkeypatch, dq)
+    op.run([x, w])
+    w.neg_()
+    assert same(op.run([x, w]), x, w, dq)
+    w[:, 1:3].fill_(3)                        # through a view
+    assert same(op.run([x, w]), x, w, dq)
+    with torch.inference_mode():              # tensors whose writes are not counted
+        v = w + 0
+        op.run([x, v])
+        v.mul_(2)
+        assert same(op.run([x, v]), x, v, dq)
+
+
+def test_views_of_the_same_weights_are_told_apart(monkeypatch):
+    x, w, dq = tensors()
+    op = operator(monkeypatch, dq)
+    assert same(op.run([x, w]), x, w, dq)
+    turned = w.transpose(2, 3)
+    assert same(op.run([x, turned]), x, turned, dq)
+    assert same(op.run([x, w]), x, w, dq)
+
+
+def test_weights_of_a_plan_stay_allocated(monkeypatch):
+    """A later tensor cannot come to lie where the weights of a kept plan were."""
+    import weakref
+    x, w, dq = tensors()
+    op = operator(monkeypatch, dq)
+    w = w.transpose(2, 3)
+    held = weakref.ref(w)
+    op.run([x, w])
+    del w
+    assert held() is not None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel", [1, 2])
+def test_attributes_and_weights_on_the_gpu(kernel):
+    x, w, dq = tensors()
+    x, w = x.cuda(), w.cuda()
+    op = ops.Conv2DQuantized(kernel)
+    configure(op, dq)
+    first = op.run([x, w])
+    w.neg_()
+    assert torch.equal(op.run([x, w]), -first)
+    turned = op.run([x, w.transpose(2, 3)])
+    assert torch.equal(turned, op.run([x, w.transpose(2, 3).contiguous()]))
+    configure(op, [2 * v for v in dq])
+    assert torch.equal(op.run([x, w]), -2 * first)
