@@ -105,17 +105,23 @@ class Quantize(Operator):
         super().__init__()
         self.field("quantize_scale", REQUIRED)
         self.scales = None
+        self._array = self._array_of = None
 
     def init(self):
         super().init()
         self.scales = [float(v) for v in np.asarray(self.get("quantize_scale"), dtype=np.float32).reshape(-1)]
-        self._scale_array = float_array(self.scales)
 
     def infer(self, inputs):
         _auto_check(len(inputs) == 1, "stack.size() == 1")
         x = inputs[0]
         _auto_check(len(self.scales) == x.shape[0], "m_quantize_scales.size() == x_tensor.sizes()[0]")
         return [("int8", tuple(x.shape))]
+
+    def _scale_array(self):
+        """The scales as the library takes them, laid out again when they are others than last time."""
+        if self.scales != self._array_of:
+            self._array, self._array_of = float_array(self.scales), list(self.scales)
+        return self._array
 
     def run(self, inputs, stream=None):
         self.infer(inputs)
@@ -126,7 +132,8 @@ class Quantize(Operator):
         y = torch.empty(x.shape, dtype=torch.int8, device=x.device)
         lib = _lib.load()
         fn = lib.tsb_quantize_f32_i8 if x.dtype == torch.float32 else lib.tsb_quantize_f64_i8
-        status = fn(x.data_ptr(), y.data_ptr(), x.numel(), self._scale_array, len(self._scale_array), _stream_ptr(stream))
+        scales = self._scale_array()
+        status = fn(x.data_ptr(), y.data_ptr(), x.numel(), scales, len(scales), _stream_ptr(stream))
         if status:
             check(status)
         return y

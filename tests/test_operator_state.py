@@ -135,3 +135,14 @@ def test_attributes_and_weights_on_the_gpu(kernel):
     assert torch.equal(turned, op.run([x, w.transpose(2, 3).contiguous()]))
     configure(op, [2 * v for v in dq])
     assert torch.equal(op.run([x, w]), -2 * first)
+
+
+def test_quantize_takes_scales_as_they_stand():
+    op = ops.Quantize()
+    op.set("quantize_scale", [1.0, 2.0])
+    op.init()
+    assert list(op._scale_array()) == [1.0, 2.0]
+    op.scales[1] = 4.0
+    assert list(op._scale_array()) == [1.0, 4.0]
+    op.scales = [3.0]
+    assert list(op._scale_array()) == [3.0]
