@@ -110,6 +110,7 @@ class Quantize(Operator):
     def init(self):
         super().init()
         self.scales = [float(v) for v in np.asarray(self.get("quantize_scale"), dtype=np.float32).reshape(-1)]
+        self._scale_array()
 
     def infer(self, inputs):
         _auto_check(len(inputs) == 1, "stack.size() == 1")
