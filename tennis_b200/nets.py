@@ -11,6 +11,9 @@ operators one by one.
 Weights are synthetic (seeded): int8 uniform in [-127,127], per-channel weight scales U(0.001,0.01), bias N(0,0.1).
 Activation scales are calibrated once on a sample batch (127 / max|activation| per tensor).
 """
+import operator
+import threading
+
 import numpy as np
 import torch
 
@@ -102,40 +105,53 @@ class QuantResNet:
         self.calibrated = False
         self.launch_log = None
         # forward(): the pass as bound library calls, laid out by the first pass after a calibration (every tensor between
-        # input and output is the network's own, so only the input's address changes)
+        # input and output is the network's own, so only the input's address changes) and again by the first pass after a change
         self.steps = None
         self.recording = None
+        self.lay_out_lock = threading.RLock()
 
-    def _step(self, call):
-        """Runs a bound library call, and notes it when a pass is being laid out."""
+    def _step(self, call, sources):
+        """Runs a bound library call, and notes it, with where its objects came from, when a pass is being laid out."""
         call(ops._stream_ptr())
         if self.recording is not None:
+            call.sources = sources
             self.recording.append(call)
 
-    def _call(self, fn, args, keep):
-        self._step(ops.Call(fn, args, keep))
+    def _call(self, fn, args, tensors, key):
+        """The same for a call that writes the buffer `key`."""
+        self._step(ops.Call(fn, args, (), tensors), ((self.buffers, key, self.buffers[key]),))
+
+    def _layer_sources(self, idx, L):
+        plan = L["plan"]
+        sources = ((self.convs, idx, L), (L, "plan", plan), (plan.__dict__, "workspace", plan.workspace), (L, "dq", L["dq"]), (L, "bias", L["bias"]))
+        return sources + ((L, "out_scale_arr", L["out_scale_arr"]),) if "out_scale_arr" in L else sources
+
+    def _buffer_sources(self, key, i8, f32):
+        sources = ((self.buffers, key + ".i8", i8),) if i8 is not None else ()
+        return sources + ((self.buffers, key + ".f32", f32),) if f32 is not None else sources
+
+    def _attributes(self):
+        return [getattr(self, name, None) for name in ("convs", "buffers", "halves", "fc_w", "fc_b", "spec", "batch", "lib", "fuse_projection",
+                                                       "fuse_concat")]
 
     def _replay(self, x, lay_out):
         """One pass: the staging quantize of x, then the bound calls; lay_out(x) is the pass as plain code, which the first
-        call records.  (A ResNet-50 pass of one image is 60 launches: 0.64 ms as plain code, which the host bounds, and 0.40 ms
-        bound, which the GPU bounds.)"""
-        fused = (self.fuse_projection, self.fuse_concat)
-        if self.steps is None or self.steps[2] != fused or self.launch_log is not None:
+        call and the first one after a change records.  (A ResNet-50 pass of one image is 57 launches: 0.64 ms as plain code, which
+        the host bounds; bound, 0.27 ms of the host, 0.04 of them the check, and 0.34 ms of the GPU, 0.31 as a graph.)"""
+        if self.steps is not None and self.launch_log is None:
+            calls, out, attributes = self.steps
+            if all(map(operator.is_, self._attributes(), attributes)):
+                self.convs[0]["plan"].quantize_input(x, self.input_scale_arr)
+                if calls.run(ops._stream_ptr()):
+                    return out
+        with self.lay_out_lock:
             self.recording = []
             try:
                 out = lay_out(x)
-                self.steps = (self.recording, out, fused)
+                self.steps = (ops.BoundCalls(self.recording), out, self._attributes())
             finally:
                 self.recording = None
             return out
-        calls, out, _ = self.steps
-        self.convs[0]["plan"].quantize_input(x, self.input_scale_arr)
-        stream = ops._stream_ptr()
-        for call in calls:
-            status = call.fn(*call.args, stream)
-            if status:
-                check(status)
-        return out
 
     # ---- buffers ------------------------------------------------------------------------------------------------
     def _i8(self, key, pixels_hw, channels):
@@ -162,7 +178,7 @@ class QuantResNet:
                                   residual=residual, activation=act, leaky=leaky, out_f32=out_f32, out_f32_layout=LAYOUT_NHWC_PAD,
                                   out_i8=out_i8, out_i8_layout=LAYOUT_NHWC_PAD,
                                   requant_scales=L["out_scale_arr"] if want_i8 else None, residual_after_activation=residual_after)
-        self._step(call)
+        self._step(call, self._layer_sources(idx, L) + self._buffer_sources(key, out_i8, out_f32))
         if self.launch_log is not None:      # layer_times(): every convolution launch of a pass, replayable
             out_bytes = (out_i8.numel() if want_i8 else 0) + (4 * self.batch * c["oh"] * c["oh"] * c["o"] if want_f32 else 0)
             in_bytes = self.batch * c["h"] * c["h"] * ops.padded_channels(c["c"]) + c["o"] * c["c"] * c["k"] * c["k"] + 8 * c["o"]
@@ -182,7 +198,7 @@ class QuantResNet:
 
         call = L["plan"].bind_projected(x_i8, S["plan"], x_proj, L["dq"], S["dq"], bias=L["bias"], shortcut_bias=S["bias"],
                                         activation=act, out_f32=out_f32, out_i8=out_i8, requant_scales=L["out_scale_arr"])
-        self._step(call)
+        self._step(call, self._layer_sources(idx, L) + self._layer_sources(idx_proj, S) + self._buffer_sources(key, out_i8, out_f32))
         if self.launch_log is not None:
             px = self.batch * c["oh"] * c["oh"]
             in_bytes = (self.batch * c["h"] * c["h"] * ops.padded_channels(c["c"]) + c["o"] * c["c"] * c["k"] * c["k"] + 8 * c["o"] +
@@ -272,7 +288,7 @@ class QuantResNet:
         c = L["spec"]
         pooled = self._i8("stem.pool", spec["stem_pooled"], c["o"])
         self._call(self.lib.tsb_maxpool_i8_nhwc, (s_i8.data_ptr(), pooled.data_ptr(), self.batch, c["oh"], c["oh"], c["o"], 3, 2, 1, 0, 1, 0),
-                   (s_i8, pooled))
+                   (s_i8, pooled), "stem.pool")
         return pooled
 
     def forward(self, x):
@@ -301,9 +317,11 @@ class QuantResNet:
                 self.buffers[key] = torch.empty((self.batch, width), dtype=torch.float32, device=self.dev)
         feat, logits = self.buffers["feat"], self.buffers["logits"]
         P = spec["final_size"] * spec["final_size"]
-        self._call(self.lib.tsb_global_avgpool_f32_nhwc, (x_f32.data_ptr(), feat.data_ptr(), self.batch, P, spec["features"]), (x_f32, feat))
+        self._call(self.lib.tsb_global_avgpool_f32_nhwc, (x_f32.data_ptr(), feat.data_ptr(), self.batch, P, spec["features"]), (x_f32, feat),
+                   "feat")
         self._call(self.lib.tsb_inner_prod_f32, (feat.data_ptr(), self.fc_w.data_ptr(), self.fc_b.data_ptr(), logits.data_ptr(), self.batch,
-                                                 spec["features"], spec["classes"]), (feat, self.fc_w, self.fc_b, logits))
+                                                 spec["features"], spec["classes"]), (feat, self.fc_w, self.fc_b, logits),
+                   "logits")
         return logits
 
     def status(self):
@@ -430,7 +448,10 @@ class QuantCSPDarknet(QuantResNet):
 
         call = p_rest.bind_concat(rest, p_first, first, L["dq"], bias=L["bias"], activation=act, leaky=leaky, out_i8=out_i8,
                                   requant_scales=L["out_scale_arr"])
-        self._step(call)
+        halves = self.halves[idx]
+        self._step(call, self._layer_sources(idx, L) + self._buffer_sources(key, out_i8, None) +
+                   ((self.halves, idx, halves), (halves, 0, p_first), (halves, 1, p_rest), (p_first.__dict__, "workspace", p_first.workspace),
+                    (p_rest.__dict__, "workspace", p_rest.workspace)))
         if self.launch_log is not None:
             px = self.batch * c["oh"] * c["oh"]
             self.launch_log.append(dict(name=c["name"] + "+concat", launch=lambda: call(ops._stream_ptr()), ops=2 * px * c["o"] * c["c"],
@@ -440,7 +461,8 @@ class QuantCSPDarknet(QuantResNet):
 
     def _concat(self, a, ca, b, cb, key, size):
         out = self._i8(key, size, ca + cb)
-        self._call(self.lib.tsb_concat_i8_nhwc, (a.data_ptr(), ca, b.data_ptr(), cb, out.data_ptr(), self.batch * size * size), (a, b, out))
+        self._call(self.lib.tsb_concat_i8_nhwc, (a.data_ptr(), ca, b.data_ptr(), cb, out.data_ptr(), self.batch * size * size), (a, b, out),
+                   key)
         return out
 
     def _scale(self, m):
