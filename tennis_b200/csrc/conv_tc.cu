@@ -580,8 +580,10 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
     const bool i8_fast = !epi.out_i8 || (epi.i8_nhwc && (epi.nscales == 1 || kp.per_sample_scale));
     if (plain && epi.out_i8 && !epi.out_f32 && i8_fast) epi_mode = kEpiI8Nhwc;
     // pixel-major fp32 tensors (block outputs and residuals of a network) where a thread owns a channel; where it owns a pixel they
-    // take the staged class, below
-    if (!epi.out_acc && (epi.out_f32 || epi.residual) && epi.f32_nhwc && i8_fast && (const void *)epi.residual != (const void *)epi.out_f32 && cfg.swap && !cfg.patch)
+    // take the staged class, below, or, in raw rows without room for it, 16-byte accesses
+    const bool nhwc_rows = v.rows && g.O % 4 == 0 && ((reinterpret_cast<uintptr_t>(epi.out_f32) | reinterpret_cast<uintptr_t>(epi.residual)) & 15) == 0;
+    if (!epi.out_acc && (epi.out_f32 || epi.residual) && epi.f32_nhwc && i8_fast && (const void *)epi.residual != (const void *)epi.out_f32 &&
+        ((cfg.swap && !cfg.patch) || nhwc_rows))
         epi_mode = kEpiNhwc;
     const int mode = cfg.patch ? kModePatch : (v.rows ? kModeRows : (cfg.split ? kModeSplit : kModeGeneral));
     // Pixel-major fp32 residual (the shortcut of a residual block, as large as the output): a tensor map over it lets the
