@@ -262,7 +262,7 @@ TSB_API int tsb_conv2d_i8_run_concat(tsb_conv_plan *plan, const int8_t *x, tsb_c
 
 /*
  * Failure detection.  Every wait inside the tensor-core kernel is bounded; a wait that runs out makes the kernel
- * write a code (1..8, which wait) into the status word at the start of the workspace, release what it holds and
+ * write a code (1..9, which wait) into the status word at the start of the workspace, release what it holds and
  * return, so the CUDA context stays usable but that run's outputs are invalid.
  *  - tsb_conv2d_i8_status: copies the word back, synchronises the stream and returns TSB_OK or
  *    TSB_ERR_DEVICE_TIMEOUT (tsb_last_error names the wait); a reported time-out is cleared again.

@@ -490,6 +490,7 @@ static const char *wait_name(int code) {
         case 6: return "MMA issuer: resident weight tile loaded";
         case 7: return "epilogue: staged tile ready";
         case 8: return "epilogue copies: staged tile written";
+        case 9: return "epilogue: partial sums of the cluster's other CTAs";
         default: return "unknown wait";
     }
 }
