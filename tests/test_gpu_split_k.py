@@ -3,6 +3,7 @@ checker bit for bit.  Shapes at the rule's edges: K of 2048 bytes and just above
 end inside a 32-channel chunk, the last pixel tile nearly empty, 64-byte K blocks, the most tiles that are still split."""
 import numpy as np
 import pytest
+import torch
 
 from conftest import same_bits
 from test_gpu_conv import run_gpu
@@ -44,6 +45,9 @@ def test_split_k(checker, geo, outputs):
               nhwc_residual=dict(rq=rq, i8_layout="nhwc", f32_layout="nhwc", residual=res), acc=dict(want_acc=True, rq=rq))[outputs]
     kw.setdefault("want_acc", False)
     got = run_gpu(x, w, (pad,) * 4, (stride,) * 2, (1, 1), dq, bias, "relu", 0.0, x_layout="nhwc", **kw)
+    if outputs == "acc":      # (whole numbers: exact in fp64 in any order)
+        sums = torch.nn.functional.conv2d(torch.from_numpy(x).double(), torch.from_numpy(w).double(), stride=stride, padding=pad)
+        assert np.array_equal(got["acc"], sums.numpy().astype(np.int32))
     if kw.get("want_f32", True):
         assert same_bits(got["f32"], y)
     if "rq" in kw:
