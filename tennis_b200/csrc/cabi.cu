@@ -380,8 +380,8 @@ int tsb_conv2d_i8_run(tsb_conv_plan *plan, const int8_t *x, int x_layout, const 
         if (st != TSB_OK) return st;
         x_tc = stage;
     }
-    // Outputs that can go through shared-memory tiles and tensor-map stores (int8 NHWC_PAD, pixel-major fp32 with or
-    // without a residual) take the configuration that sets the tiles' shared memory aside.
+    // Outputs that go through shared-memory tiles and tensor-map stores (pixel-major fp32 with or without a residual, with or
+    // without int8 NHWC_PAD) take the configuration that sets the tiles' shared memory aside.
     if (plan->stg_valid && tc::wants_staging(plan->view, epi)) {
         if (plan->map_a_stg_ptr != x_tc) {
             st = tc::encode_activation_map(plan->view, plan->cfg_stg, x_tc, &plan->map_a_stg);
@@ -413,7 +413,7 @@ int tsb_conv2d_i8_run(tsb_conv_plan *plan, const int8_t *x, int x_layout, const 
     return tc::launch_conv_tc(plan->view, plan->cfg, plan->map_a, plan->map_b, x_tc, epi, plan->status_word ? plan->status_word : static_cast<int *>(workspace), stream);
 }
 
-// Two convolutions in one launch (conv_tc.cu, DUAL instances).  concat == false: `shortcut` is a projection whose dequantized
+// Two convolutions in one launch (conv_tc_kernel.cuh, DUAL instances).  concat == false: `shortcut` is a projection whose dequantized
 // (+ bias) result is the residual of `plan`.  concat == true: `shortcut` convolves the leading channels of a concatenated
 // input and `plan` the rest; both sum into one accumulator.
 static int run_pair(tsb_conv_plan *plan, const int8_t *x, tsb_conv_plan *shortcut, const int8_t *x_shortcut,
@@ -479,7 +479,7 @@ int tsb_conv2d_i8_run_concat(tsb_conv_plan *plan, const int8_t *x, tsb_conv_plan
     return run_pair(plan, x, first, x_first, nullptr, nullptr, epilogue, tile_channels, workspace, workspace_bytes, stream, true);
 }
 
-// what each code of the status word means (the kernel's bounded waits, conv_tc.cu)
+// what each code of the status word means (the kernel's bounded waits, conv_tc_kernel.cuh)
 static const char *wait_name(int code) {
     switch (code) {
         case 1: return "producer: pipeline stage free";

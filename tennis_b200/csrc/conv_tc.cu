@@ -147,14 +147,15 @@ static uint32_t staged_bytes(int tiles) { return tiles ? kQuads * ((uint32_t)til
 // bytes of K from which on a layer of few tiles is split
 constexpr int kSplitMinK = 2048;
 
-// tiles: fp32 tiles per quad of the staged epilogue, 0: not staged
+// tiles_per_quad: fp32 tiles per quad of the staged epilogue, 0: not staged
 static Config plan_config(const View &v, const Tuning &tune, int sm_count, int orientation, int tiles_per_quad) {
     const ConvGeom &g = v.g;
     Config c;
     c.bk = (g.Cp % 128 == 0) ? 128 : 64;
     const int64_t M = (int64_t)g.N * g.OH * g.OW;
     uint32_t stg_bytes = staged_bytes(tiles_per_quad), budget = kSmemBudget - stg_bytes;
-    // An MMA instruction costs the same 128 cycles for any N up to 256, so N should be 256 whenever possible.
+    // An MMA instruction costs the issuing warp 77-115 cycles whatever its N (the tensor core 128 at N = 256, 64 at 128, 48 at 64), so N should
+    // be 256 whenever possible.
     // Normal orientation: 128 pixels on M, up to 256 output channels on N.  Swapped orientation: channels on M,
     // 256 (or 128) pixels on N -- it halves the MMA count of narrow layers but its epilogue (one channel per thread)
     // is dearer, so it is taken where it measured faster: multi-tap filters with at most 64 output channels.
@@ -543,7 +544,7 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
     kp.d_P = FastDiv((uint32_t)kp.P); kp.d_OW = FastDiv((uint32_t)kp.OW);
     kp.d_m_tiles = FastDiv((uint32_t)cfg.num_m_tiles); kp.d_n_tiles = FastDiv((uint32_t)cfg.num_n_tiles);
     kp.d_segs = FastDiv((uint32_t)std::max(1, v.rows_segs)); kp.d_OH = FastDiv((uint32_t)g.OH); kp.d_dh = FastDiv((uint32_t)g.dh);
-    kp.per_sample_scale = (epi.nscales > 1 && epi.nscales == g.N && epi.group_len == (uint32_t)(g.O * g.OH * g.OW)) ? 1 : 0;
+    const bool per_sample = epi.nscales > 1 && epi.nscales == g.N && epi.group_len == (uint32_t)(g.O * g.OH * g.OW);    // scale index = image index
     kp.status = status_word;
 #ifdef TSB_ENABLE_TRACE
     kp.trace = g_trace;
@@ -577,7 +578,7 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
     // ... and with an fp32 NCHW residual (a shortcut folded into the convolution by the graph rewrite), where a thread owns a pixel
     if (!cfg.swap && !epi.out_acc && epi.residual && epi.out_f32 && !epi.f32_nhwc && !epi.out_i8 && (const void *)epi.residual != (const void *)epi.out_f32)
         epi_mode = kEpiF32Nchw;
-    const bool i8_fast = !epi.out_i8 || (epi.i8_nhwc && (epi.nscales == 1 || kp.per_sample_scale));
+    const bool i8_fast = !epi.out_i8 || (epi.i8_nhwc && (epi.nscales == 1 || per_sample));
     if (plain && epi.out_i8 && !epi.out_f32 && i8_fast) epi_mode = kEpiI8Nhwc;
     // pixel-major fp32 tensors (block outputs and residuals of a network) where a thread owns a channel; where it owns a pixel they
     // take the staged class, below, or, in raw rows without room for it, 16-byte accesses
@@ -595,7 +596,7 @@ int launch_conv_tc(const View &v, const Config &cfg, const CUtensorMap &map_a, c
         load_driver() == TSB_OK) {
         cuuint64_t dims[2] = {(cuuint64_t)g.O, (cuuint64_t)kp.M_total};
         cuuint64_t strides[1] = {(cuuint64_t)g.O * 4};
-        cuuint32_t box[2] = {cfg.swap ? (cuuint32_t)std::min(g.O, kBM) : 32u, cfg.swap ? 32u : (cuuint32_t)kBM};
+        cuuint32_t box[2] = {(cuuint32_t)std::min(g.O, kBM), 32u};
         cuuint32_t estr[2] = {1, 1};
         if (g_encode_tiled(&map_r, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(epi.residual), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

@@ -1,4 +1,4 @@
-// Host interface of the tcgen05 implicit-GEMM convolution (conv_tc.cu).
+// Host interface of the tcgen05 implicit-GEMM convolution (host side conv_tc.cu, kernel conv_tc_kernel.cuh).
 #pragma once
 
 #include <cuda.h>

@@ -6,16 +6,19 @@
 //               are resolved by the tensor map, nothing is materialised in memory
 //   B operand   weights, int8 [O][KH][KW][Cp]; plain 2-D TMA tiles of BN x BK
 //   MMA         tcgen05.mma kind::i8, 128 x BN x 32 per instruction, int32 accumulators in tensor memory,
-//               issued by one thread; two accumulator buffers so the epilogue of tile i overlaps the
-//               main loop of tile i+1
+//               issued by two warps on alternate tiles; up to four accumulator buffers, so the epilogue of a
+//               tile overlaps the main loops of the next ones
 //   epilogue    sixteen warps read the accumulators with tcgen05.ld and apply dequantize / bias / residual /
-//               activation / requantize in registers, then store fp32 (NCHW or NHWC) and/or int8
+//               activation / requantize in registers, then store fp32 (NCHW or NHWC) and/or int8, or hand
+//               them to four copy warps in shared-memory tiles (staged class)
 //
-// Warp roles in a CTA of 576 threads: warp 0 = TMA producer, warp 1 = tensor-memory owner + MMA issuer,
-// warps 2..17 = epilogue.  The kernel is persistent: gridDim.x CTAs walk the tile list with stride gridDim.x.
+// Warp roles in a CTA of 608 threads (736 in the staged class): warp 0 = TMA producer, warps 1 and 2 = MMA issuers (warp 1
+// owns tensor memory), warps 3..18 = epilogue, warps 19..22 = the staged class's copies.  The kernel is persistent:
+// gridDim.x CTAs walk the tile list with stride gridDim.x, or, with resident weights, each a range of it.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out records a code in *status, raises a CTA-wide
 // abort flag and all roles fall through to the common exit, where tensor memory is released.
+// (barrier.cluster.wait, in split-K, has no bound of its own: see there.)
 #pragma once
 
 #include "conv_common.cuh"
@@ -198,10 +201,9 @@ __device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// The same, executed only when `on` is non-zero -- a predicated instruction, not a branch.  The issuing thread runs
-// alone in its warp and pays tens of cycles for every branch or dependent instruction, so its MMA sequences are
-// straight-line code in which inactive slots (a filter row outside the image, a k block beyond the group) are switched
-// off by predicate.
+// The same, executed only when `on` is non-zero -- a predicated instruction, not a branch.  What an issuing warp spends between two MMAs is
+// not hidden, so its MMA sequences are straight-line code in which inactive slots (a filter row outside the image, a tap beyond
+// the filter) are switched off by predicate.
 __device__ __forceinline__ void mma_i8_if(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t on) {
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
@@ -234,39 +236,14 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const int (&v)[32]) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Shared-memory matrix descriptor of a K-major tile whose rows are one swizzle span (BK bytes) wide:
-// 8-row groups are 8*BK bytes apart (stride byte offset); version 1; swizzle 128B (2) or 64B (4).
-template <int BK>
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-    constexpr uint64_t layout = BK == 128 ? 2 : (BK == 64 ? 4 : 6);
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)1 << 16;                       // leading byte offset: unused for swizzled K-major
-    d |= (uint64_t)((8 * BK) >> 4) << 32;         // stride byte offset
-    d |= (uint64_t)1 << 46;                       // descriptor version of this architecture
-    d |= layout << 61;
-    return d;
-}
-
-// The same with a run-time stride between 8-row groups and a start that need not be 1024-byte aligned (patch mode).
-// The swizzle is a function of the absolute shared-memory address (measured: any 128-byte-aligned start and any group
-// stride read back what a tensor-map copy with the same swizzle wrote; the base-offset field stays 0).
-template <int BK>
-__device__ __forceinline__ uint64_t smem_desc_strided(uint32_t saddr, uint32_t group_stride_bytes) {
-    constexpr uint64_t layout = BK == 128 ? 2 : (BK == 64 ? 4 : 6);
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(group_stride_bytes >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= layout << 61;
-    return d;
-}
-
-// The same descriptors split for the issuing thread's inner loops: everything but the 14-bit start-address field is
-// loop-invariant, so a loop keeps the invariant part in a register and ORs in (address >> 4) -- shared-memory addresses
-// stay below 2^18, so the field never overflows into its neighbours, and stepping along K inside a swizzle span or to
-// another filter tap is a plain add on that field.
+// Shared-memory matrix descriptor of a K-major tile whose rows are one swizzle span (BK bytes) wide: 8-row groups are
+// group_stride_bytes apart (8*BK in a tile that is packed; more under a patch, whose rows a window skips); leading byte offset unused;
+// version 1; swizzle 128B (2) or 64B (4).  The swizzle is a function of the absolute shared-memory address (measured: any
+// 128-byte-aligned start and any group stride read back what a tensor-map copy with the same swizzle wrote; the base-offset
+// field stays 0), so a start need not be 1024-byte aligned.
+// Everything but the 14-bit start-address field is loop-invariant, so a loop keeps the invariant part in a register and ORs in
+// (address >> 4) -- shared-memory addresses stay below 2^18, so the field never overflows into its neighbours, and stepping along K
+// inside a swizzle span or to another filter tap is a plain add on that field.
 template <int BK>
 __device__ __forceinline__ constexpr uint64_t smem_desc_hi(uint32_t group_stride_bytes) {
     return ((uint64_t)1 << 16) | ((uint64_t)(group_stride_bytes >> 4) << 32) | ((uint64_t)1 << 46) |
@@ -303,12 +280,12 @@ __device__ __forceinline__ constexpr uint32_t instr_desc() {
 // epilogue: 32 accumulator columns of one output pixel (one thread) at a time
 // ---------------------------------------------------------------------------------------------------------
 // Which one a launch takes is a template parameter of the kernel (EPI): an instance holds the code of one class only.  With all
-// classes in one kernel every class paid for the others: 700 bytes of spills in all of them (now none, 340 in the staged class),
-// and a variant more cost the layers that never ran it 3-8 %.  Measured with the classes apart: the five sweep layers at batch 32
-// 126 -> 115 us, a ResNet-50 pass of 64 images 1.42 -> 1.35 ms.
+// classes in one kernel every class paid for the others: 700 bytes of spills in all of them (now at most 32, 48 in the
+// staged class, 304 in the pixel-major one of raw rows), and a variant more cost the layers that never ran it 3-8 %.  Measured with the
+// classes apart: the five sweep layers at batch 32 126 -> 115 us, a ResNet-50 pass of 64 images 1.42 -> 1.35 ms.
 constexpr int kEpiGeneric = 0;   // any combination of outputs, element by element
 constexpr int kEpiF32Nchw = 1;   // fp32 NCHW output only (the operator's own output)
-constexpr int kEpiI8Nhwc = 2;    // requantized int8 NHWC_PAD output only, half-away rounding, one scale per sample
+constexpr int kEpiI8Nhwc = 2;    // requantized int8 NHWC_PAD output only, one scale for the batch (half to even) or per image (half away from zero)
 constexpr int kEpiNhwc = 3;      // fp32 [N][P][O] residual in and/or fp32 [N][P][O] out and/or int8 NHWC_PAD out, from registers (swapped orientation;
                                  // raw rows whose weights leave no room for the staged class)
 constexpr int kEpiStaged = 4;    // the same outputs through shared-memory tiles and tensor-map loads / stores (normal orientation)
@@ -773,7 +750,6 @@ struct KernelParams {
     int Cp;          // channels of the staged input per filter tap
     int num_m_tiles, num_n_tiles;   // pixel tiles, channel tiles
     FastDiv d_P, d_OW, d_m_tiles, d_n_tiles, d_segs, d_OH, d_dh;   // dividers by P, OW, num_m_tiles, num_n_tiles, rows_segs, rows_OH, dh
-    int per_sample_scale;  // requantize: scale index = image index
     int a_tiled;           // activations are a plain [M][Cp] matrix (1x1, stride 1, no padding): 2-D tile loads
     // shared-memory plan (bytes from the 1024-aligned base)
     int stages;            // pipeline stages (<= kMaxStages)
@@ -804,8 +780,8 @@ struct KernelParams {
     uint32_t patch_bytes;                     // bytes of one patch (one channel block)
     int OH;
     FastDiv d_tiles_w, d_tiles_hw;
-    int res_prefetch;      // the residual tensor has a tensor map (map_r): the epilogue prefetches its boxes into L2 two
-                           // chunks ahead of the loads, so that those find the data on chip
+    int res_prefetch;      // swapped orientation: the residual tensor has a tensor map (map_r), by which the epilogue prefetches boxes of it into
+                           // L2 two chunks ahead of the registers' loads, so that those find the data on chip
     int *status;     // device word: 0 ok, else the code of the wait that ran out
     unsigned long long *trace;  // profiling builds: timeline of CTA 0, 8 stamps per tile, 32 tiles (null otherwise)
 };
@@ -890,10 +866,11 @@ __host__ __device__ constexpr uint32_t num_barriers(int stages) { return 2u * (u
 
 // PIX pixels x CH channels per tile.  Normal orientation: the pixel tile is the MMA's A operand (M = 128 pixels), the
 // weight tile its B operand (N = BN channels).  Swapped orientation: the weight tile is A (M = 128 channels, rows
-// beyond O zero-filled by the tensor map) and the pixel tile is B (N = BN pixels).  An MMA instruction takes the same
-// 128 cycles whatever its N, so layers with at most 128 output channels run swapped: N = 256 pixels fills the
-// instruction where N = O would leave it half or three-quarters empty.
-// MODE: how activations reach shared memory -- kModeGeneral (im2col or plain 2-D tile loads), kModeRows (raw-row), kModePatch.
+// beyond O zero-filled by the tensor map) and the pixel tile is B (N = BN pixels).  An MMA instruction takes the tensor core 128 cycles at
+// N = 256, 64 at 128 and 48 at 64, but the issuing warp 77-115 whatever its N, so narrow multi-tap layers run swapped: N = 256 pixels
+// where N = O would leave the tensor core waiting.
+// MODE: how activations reach shared memory -- kModeGeneral (im2col or plain 2-D tile loads), kModeSplit (the same, K shared out over a
+// cluster), kModeRows (raw-row), kModePatch.
 // A compile-time parameter: the role loops of each mode stay short and keep their registers.
 template <int BN, int BK, bool SWAP, int MODE, int EPI, bool DUAL>
 __global__ void __launch_bounds__(cta_threads(EPI), 1)
@@ -1170,7 +1147,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
     } else if (warp <= kIssuers) {
         // ------------------------------------------------------------------ MMA issuers
-        // One thread feeds the tensor core, but the whole warp walks the tiles: an MMA takes its descriptors from uniform registers,
+        // One thread at a time feeds the tensor core, but its whole warp walks the tiles: an MMA takes its descriptors from uniform registers,
         // and where the code is known to run converged (waits that answer through a vote, the issuing lane chosen by elect.sync) they are
         // computed there; a lane that runs alone moves every operand over instead.  64 images: ResNet-50 1.20 -> 1.15 ms, 8 images
         // 0.452 -> 0.424 ms; CSPDarknet53, 16 images 2.71 -> 2.58 ms, one image 0.609 -> 0.570 ms.
@@ -1567,7 +1544,9 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             decode(local, m_tile, n_tile);
             const int o_base = n_tile * CH;
             const int slot = DUAL ? 2 * acc : acc;          // first accumulator buffer of this tile
-            if constexpr (SPLIT) cluster_wait();    // ... and those of the other CTAs, to which partial sums will go
+            // ... and those of the other CTAs, to which partial sums will go.  (A barrier without a bound: the CTAs of a cluster start together and
+            // arrive before any other wait than that for tensor memory, which a kernel before this one gives back when it ends.)
+            if constexpr (SPLIT) cluster_wait();
             float *t_dq = table + (DUAL ? 2 * group : group) * 2 * BN, *t_bias = t_dq + BN;
             if (!SWAP && n_tile != table_n) {
                 // this group's table of per-channel scales and biases: rebuilt only when the channel tile changes (never, for
@@ -1938,7 +1917,7 @@ conv_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     __syncthreads();
     if constexpr (SPLIT) {
         // Nobody may write to, or arrive in, a CTA that has left.  One that has its partial sums gets no more of either; one that gave up
-        // stays until the others have left or given up (threads that have exited count as arrived).
+        // stays until the others have left or given up (threads that have exited count as arrived), which their own bounded waits see to.
         if (warp < kEpiWarp0 || warp >= kCopyWarp0) cluster_wait();     // (the epilogue warps have done so above)
         if (*abort_flag) { cluster_arrive(); cluster_wait(); }
     }
