@@ -38,11 +38,23 @@ if ROOT not in sys.path:
 TRAFFIC_RECORD = os.path.join(ROOT, "profiles", "conv_i8_tc_kernel_config1.md")
 
 
-def ncu_traffic_record():
-    """DRAM bytes per convolution launch from the ncu capture summarised under profiles/, valid only for the kernel source
-    it was captured with: the summary carries the SHA-256 of tennis_b200/csrc/conv_tc_kernel.cuh at capture time.  Returns
-    (bytes or None, stale flag, note)."""
+# what decides the DRAM traffic of a convolution launch: the kernel, and the host side that picks its load mode, tiles and tensor maps
+TRAFFIC_SOURCES = [os.path.join(ROOT, "tennis_b200", "csrc", f) for f in
+                   ("conv_tc_kernel.cuh", "conv_tc.cu", "conv_tc.h", "conv_common.cuh", "common.cuh", "cabi.cu")]
+
+
+def traffic_sources_sha256():
     import hashlib
+    digest = hashlib.sha256()
+    for path in TRAFFIC_SOURCES:
+        digest.update(open(path, "rb").read())
+    return digest.hexdigest()
+
+
+def ncu_traffic_record():
+    """DRAM bytes per convolution launch from the ncu capture summarised under profiles/, valid only for the sources it was
+    captured with: the summary carries the SHA-256 of TRAFFIC_SOURCES at capture time.  Returns (bytes or None, stale flag,
+    note)."""
     import re
     try:
         text = open(TRAFFIC_RECORD).read()
@@ -50,12 +62,12 @@ def ncu_traffic_record():
         m_hash = re.search(r"conv_tc_sha256\s*=\s*([0-9a-f]{64})", text)
         if not m_bytes or not m_hash:
             return None, True, "no traffic record in %s" % os.path.relpath(TRAFFIC_RECORD, ROOT)
-        now = hashlib.sha256(open(os.path.join(ROOT, "tennis_b200", "csrc", "conv_tc_kernel.cuh"), "rb").read()).hexdigest()
-        if now != m_hash.group(1):
-            return None, True, "the kernel source changed since the ncu capture in %s" % os.path.relpath(TRAFFIC_RECORD, ROOT)
+        if traffic_sources_sha256() != m_hash.group(1):
+            return None, True, "the kernel's sources changed since the ncu capture in %s" % os.path.relpath(TRAFFIC_RECORD, ROOT)
         return float(m_bytes.group(1)), False, "ncu capture summarised in %s" % os.path.relpath(TRAFFIC_RECORD, ROOT)
     except OSError as e:
         return None, True, repr(e)
+
 
 METRIC = "int8_conv_tops"
 UNIT = "TOPS"
