@@ -11,7 +11,7 @@ data-path collective, only the barrier and the max-over-ranks of the device time
 The ten launches of a step are captured once in a CUDA graph and replayed inside the timed region (--eager times the
 plain launches); every step is preceded by a 256 MiB write that flushes L2 and is timed with its own pair of CUDA events.
 
-Prints ONE JSON line (rank 0):
+Prints ONE JSON line (rank 0), and the two networks' per-layer tables on stderr:
   value        int8 TOPS of the whole job, inputs resident in HBM, device time from CUDA events
   e2e          the same metric through the host-buffer C-ABI call (H2D of the fp32 input and D2H of the fp32
                output inside the timed region, pinned host memory)
@@ -213,6 +213,26 @@ class ClockSampler(threading.Thread):
             d["error"] = self.error
         return d
 
+
+
+def emit(line):
+    """The result as one JSON line on stdout.  The networks' per-layer tables (121 rows, two thirds of the whole) go to stderr, a line
+    each: with them the line was longer than those who read it took."""
+    for name in ("resnet50", "cspdarknet53"):
+        if isinstance(line.get(name), dict) and "layers" in line[name]:
+            rest = dict(line[name])
+            print("%s layers %s" % (name, json.dumps(rest.pop("layers"))), file=sys.stderr, flush=True)
+            line = dict(line, **{name: rest})
+    print(json.dumps(short(line)), flush=True)
+
+
+def short(value):
+    """Seven digits of every number."""
+    if isinstance(value, dict):
+        return {k: short(v) for k, v in value.items()}
+    if isinstance(value, (list, tuple)):
+        return [short(v) for v in value]
+    return float("%.7g" % value) if isinstance(value, float) else value
 
 
 def layer_table(times, peaks):
@@ -1158,7 +1178,7 @@ def run_ours(args):
                     "sample": "%d images of each of the 5 layers on each of %d worker(s); %.1f s" % (images, workers, time.perf_counter() - t0)}
             except Exception as e:
                 line["cpu_baseline"] = {"value": None, "unit": UNIT, "cores": 0, "kind": "port", "sample": "failed: %r" % (e,)}
-        print(json.dumps(line))
+        emit(line)
     if world > 1:
         dist.destroy_process_group()
 

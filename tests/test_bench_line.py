@@ -1,4 +1,5 @@
-"""The bench's records: when the captured DRAM traffic still counts."""
+"""The bench's records: when the captured DRAM traffic still counts, and what goes into the result line."""
+import json
 import shutil
 
 import bench
@@ -21,3 +22,13 @@ def test_traffic_record_is_stale_once_a_source_that_decides_traffic_changes(tmp_
         assert bench.ncu_traffic_record()[:2] == (None, True)
         open(path, "w").write(before)
     assert bench.ncu_traffic_record()[:2] == (1e6, False)
+
+
+def test_the_result_is_one_line_without_the_networks_tables(capsys):
+    rows = [{"name": "s5b4.conv2", "shape": "3x3 512->512 @19", "outputs": "residual+f32+i8", "us": 27.11, "frac": 0.2993}] * 72
+    bench.emit({"metric": "m", "value": 1 / 3, "n": 123456789, "layers": rows[:5], "resnet50": {"ms": 1.0, "layers": rows}, "cspdarknet53": {"ms": 2.0, "layers": rows}})
+    out, err = capsys.readouterr()
+    line = json.loads(out)
+    assert out.count("\n") == 1 and line["value"] == 0.3333333 and line["n"] == 123456789 and line["resnet50"] == {"ms": 1.0} and line["cspdarknet53"] == {"ms": 2.0} and len(line["layers"]) == 5
+    tables = dict((l.split(" layers ", 1)[0], json.loads(l.split(" layers ", 1)[1])) for l in err.splitlines())
+    assert tables == {"resnet50": rows, "cspdarknet53": rows}
