@@ -18,7 +18,7 @@ def dequantize_scales(weight_scales, bn, input_scale):
 
 
 def resnet_forward(spec, params, scales, x, chk):
-    """x: fp32 NCHW numpy batch (more than one sample, so that quantize takes its one-scale-per-sample branch).
+    """x: fp32 NCHW numpy batch (a batch of one takes quantize's one-scale rounding, a larger one its one-scale-per-sample branch).
     Returns (int8 output of every bottleneck block, fp32 output of the last block, logits)."""
     n = x.shape[0]
     convs, P = spec["convs"], params["convs"]

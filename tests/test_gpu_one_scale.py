@@ -1,5 +1,5 @@
 """Requantize with one scale (a batch of one: half to even, but half away from zero in the tensor's last count % 8 elements) and
-channel / pixel counts that end inside a 32-column chunk, through every epilogue of the tensor-core kernel, against the CPU
+channel / pixel counts that end inside a 32-column chunk, through every epilogue of a plain convolution, against the CPU
 checker: bit for bit.  Scales and biases are powers of two, so that about one value in eight is an exact tie."""
 import numpy as np
 import pytest
